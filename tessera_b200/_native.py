@@ -22,7 +22,7 @@ _lib = None
 
 def build() -> str:
     """Compile libtmpm.so with nvcc (cross-compiles without a GPU)."""
-    subprocess.run(["make", "-s", "-C", os.path.join(_HERE, "csrc"), "-j4"], check=True)
+    subprocess.run(["make", "-s", "-C", os.path.join(_HERE, "csrc"), "-j8"], check=True)
     return LIB_PATH
 
 

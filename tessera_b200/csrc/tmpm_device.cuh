@@ -545,6 +545,17 @@ __device__ __forceinline__ V3f contact_velocity(const DevObstacle &o, V3f point,
     return surface + tangent * sc;
 }
 
+__device__ __forceinline__ void add_reaction(double *reactions, int oi, V3f center, V3f point, V3f impulse) {
+    V3f ang = cross(point - center, impulse);
+    double *r = reactions + 6 * oi;
+    atomicAdd(r + 0, static_cast<double>(impulse.x));
+    atomicAdd(r + 1, static_cast<double>(impulse.y));
+    atomicAdd(r + 2, static_cast<double>(impulse.z));
+    atomicAdd(r + 3, static_cast<double>(ang.x));
+    atomicAdd(r + 4, static_cast<double>(ang.y));
+    atomicAdd(r + 5, static_cast<double>(ang.z));
+}
+
 // RigidObstacle::cpic_side for a triangle prism (obstacle.rs:343-370; the
 // reference shader's f32 form with its 1e-5 barycentric margin, gpu.wgsl:82-102):
 // distance to the triangle's plane and the side, when the point projects into

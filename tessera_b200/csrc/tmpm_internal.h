@@ -37,6 +37,9 @@ constexpr uint32_t kStatusResident = 1u;  // CFL, escape, irregular F, non-finit
 constexpr uint32_t kStatusCapacity = 2u;  // hash table or block pool exhausted -> Capacity
 constexpr uint32_t kStatusTimeout = 4u;   // a bounded device wait gave up -> Readback
 
+// A set bit makes later kernels of the batch skip their work.
+constexpr uint32_t kFatal = kStatusCapacity | kStatusTimeout | kStatusResident;
+
 // GPU material codes (the reference shader's codes, gpu.rs:1171-1276).
 constexpr int kMatNeoHookean = 1;
 constexpr int kMatFluid = 2;
@@ -233,6 +236,34 @@ struct ForkJoin {
     cudaStream_t side;
     cudaEvent_t fork, join;
 };
+
+// PLASTIC selects the variant that carries plastic state (snow, sand, NH sand);
+// scenes without plastic materials run the leaner variant.  VARIANT selects
+// kPlain (one scene without obstacles, parameters from the kernel parameters),
+// kPlainObst (the same with rigid obstacles), kMulti (a multi-scene batch,
+// which has no obstacles: each particle reads its scene's parameters from the
+// scene table, scene = class namespace >> kSceneShift, and takes part only in
+// the substeps its scene advances in this batch) or kCpic (one scene with
+// obstacles whose grid namespace includes CPIC side masks).  Each costs
+// registers only where used: the obstacle contact calls an out-of-line
+// surface function, and with that call in the kernel the register allocator
+// kept ~500 more bytes per thread in local memory on every particle's path
+// (80 registers: 172 bytes of spill stores against 28 without it), which cost
+// the obstacle-free dam break ~10 % of its fused transfer time.
+enum Variant : int { kPlain = 0, kMulti = 1, kCpic = 2, kPlainObst = 3 };
+constexpr bool has_obstacles(int variant) { return variant == kCpic || variant == kPlainObst; }
+
+
+// Per-variant transfer launchers (tmpm_transfer_*.cu); with `fj` the fused
+// transfer runs in two tiers.
+template <int V>
+void launch_transfer_variant(int mode, const ParticleSoA &P, int n, const DevClass *classes, const GridTable &cur,
+                             const GridTable &next, const SimParams &sp, const DevObstacle *obstacles,
+                             const float *planes, double *reactions, uint32_t *status, int *cache,
+                             cudaStream_t stream, const ForkJoin *fj);
+// Load the kernels of every tuner candidate of a variant.
+template <int V>
+void preload_transfer_variant();
 
 // Launchers (tmpm_kernels.cu).  All run on `stream`.
 // `cur` and `next` share one hash table (block ids are stable within a batch)

@@ -1,0 +1,7 @@
+// tmpm_transfer_multi.cu -- transfer kernels: multi-scene batches.
+#include "tmpm_transfer.cuh"
+
+namespace tmpm {
+TMPM_TRANSFER_VARIANT(kMulti)
+template void preload_transfer_variant<kMulti>();
+}  // namespace tmpm
