@@ -288,22 +288,48 @@ __device__ __forceinline__ float pow2_scale(float total) {
 // two per axis, slot (qx << 2) | (qy << 1) | qz for block (b >> BS) + q.  Each
 // thread looks up (or, INSERT, finds or inserts) the distinct ones and stores
 // the ids at ids[slot * THREADS], the unreached slots -1.
+//
+// Bound by latency: a CTA on this path is one of a few beside the fast kernel,
+// and a lookup is a key load and then a value load.  So the first slot of every
+// reached block is read at once, key and value together (one memory round trip
+// instead of up to sixteen); only a block whose first slot holds another key,
+// or whose id is not published yet, goes through the probing functions.  An id
+// read here without acquire is safe to use: an id is written once, after its
+// key, and the pools' nodes are zeroed before the table's first insert.
 template <int THREADS, int BS, bool INSERT>
 __device__ __forceinline__ void stencil_blocks(const GridTable &g, const int b[3], uint32_t ns, int *ids,
                                                uint32_t *status) {
     const int g0 = b[0] >> BS, g1 = b[1] >> BS, g2 = b[2] >> BS;
     const int e0 = ((b[0] + 2) >> BS) - g0, e1 = ((b[1] + 2) >> BS) - g1, e2 = ((b[2] + 2) >> BS) - g2;
+    unsigned long long found[8];
+    uint32_t val[8];
+#pragma unroll
     for (int q = 0; q < 8; ++q) {
         const int qx = q >> 2, qy = (q >> 1) & 1, qz = q & 1;
-        int id = -1;
+        found[q] = kEmptyKey;
+        val[q] = kPendingId;
         if (qx <= e0 && qy <= e1 && qz <= e2) {
-            const unsigned long long key = block_key(g0 + qx, g1 + qy, g2 + qz, ns);
-            if constexpr (INSERT)
-                id = find_or_insert_block(g, key, make_int4(g0 + qx, g1 + qy, g2 + qz, static_cast<int>(ns)), status);
-            else
-                id = lookup_block(g, key);
+            const uint32_t slot = hash_slot(block_key(g0 + qx, g1 + qy, g2 + qz, ns), g.mask);
+            found[q] = __ldcg(g.keys + slot);
+            val[q] = __ldcg(g.vals + slot);
         }
-        ids[q * THREADS] = id;
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const int qx = q >> 2, qy = (q >> 1) & 1, qz = q & 1;
+        const unsigned long long key = block_key(g0 + qx, g1 + qy, g2 + qz, ns);
+        ids[q * THREADS] = found[q] == key && val[q] < kInvalidId ? static_cast<int>(val[q]) : -1;
+    }
+#pragma unroll 1
+    for (int q = 0; q < 8; ++q) {
+        const int qx = q >> 2, qy = (q >> 1) & 1, qz = q & 1;
+        if (qx > e0 || qy > e1 || qz > e2 || ids[q * THREADS] >= 0) continue;
+        const unsigned long long key = block_key(g0 + qx, g1 + qy, g2 + qz, ns);
+        if constexpr (INSERT)
+            ids[q * THREADS] =
+                find_or_insert_block(g, key, make_int4(g0 + qx, g1 + qy, g2 + qz, static_cast<int>(ns)), status);
+        else
+            ids[q * THREADS] = lookup_block(g, key);
     }
 }
 // The slot (stencil_blocks) of the block holding cell (cx, cy, cz) of the
@@ -471,7 +497,10 @@ __device__ __forceinline__ void transfer_chunk(TMPM_TRANSFER_PARAMS, const int c
         // very positions (ids are stable within a batch), so normally no box
         // reduction and no hash lookup is needed.  A record that does not
         // cover every particle sends the CTA through the general path.
-        bool use_cache = cc[0] == record_tag(sp.step_index);
+        // The negative tag says that the P2G took the direct path: so does the
+        // gather, without another box reduction.
+        const int record = cc[0];
+        bool use_cache = record == record_tag(sp.step_index);
         if constexpr (FAST) {
             if (!use_cache) return;  // on the no-record list (CTA-uniform)
         }
@@ -495,6 +524,9 @@ __device__ __forceinline__ void transfer_chunk(TMPM_TRANSFER_PARAMS, const int c
                 bx.nbt = cc[15];
                 bx.ok = 1;
                 tile_strides(bx.dim[1], bx.dim[2], bx.s1, bx.s2);
+            } else if (!FAST && record == -record_tag(sp.step_index)) {
+                bx.ok = 0;
+                bx.color = 0;
             } else if constexpr (!FAST) {
                 reduce_box<THREADS, BS>(g2p_on, b, ns, s_red, s_box);
                 bx = s_box;
@@ -959,7 +991,7 @@ __device__ __forceinline__ void transfer_chunk(TMPM_TRANSFER_PARAMS, const int c
         }
     } else {
         if (threadIdx.x == 0) {
-            cc[0] = 0;
+            cc[0] = -record_tag(sp.step_index + 1);
             if (sp.defer) defer_push(sp, 2 + ((sp.step_index + 1) & 1), chunk);
         }
         if (active) {
