@@ -643,6 +643,10 @@ struct TmpmBatch {
         if (sp.defer) cudaMemsetAsync(sp.defer, 0, sizeof(uint32_t) * kDeferHeader, stream);
         SimParams sp0 = sp;
         sp0.step_index = -1;
+        if (launch_small_segment(dst, n, dclasses.ptr, g[1], g[0], sp0, nullptr, nullptr, nullptr, status.ptr,
+                                 cta_cache.ptr, static_cast<int>(steps), sp.defer ? sp.defer + kBarrierWord : nullptr,
+                                 stream))
+            return;
         launch_transfer(kModeP2G, dst, n, dclasses.ptr, g[1], g[0], sp0, nullptr, nullptr, nullptr, status.ptr,
                         cta_cache.ptr, stream);
         for (uint32_t s = 0; s < steps; ++s) {

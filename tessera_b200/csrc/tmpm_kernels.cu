@@ -10,16 +10,13 @@
 // which alone writes velocity and the affine matrix back to HBM.  The transfer
 // kernels are in tmpm_transfer.cuh.
 
-#include "tmpm_device.cuh"
+#include "tmpm_grid.cuh"
 
 namespace tmpm {
 
 namespace {
 
-// Grid update over all allocated blocks; also zeroes those blocks in the other pool.
-// MULTI: each block takes its scene's parameters from the scene table
-// (scene = block namespace >> kSceneShift).  Blocks have edge 2^BS cells.
-// OBST: the scene has rigid obstacles (a batch never has).
+// Grid update (grid_nodes) as a kernel of its own.
 template <bool MULTI, int BS, bool OBST>
 __global__ void __launch_bounds__(256) k_grid(GridTable g, GridTable nxt, SimParams sp,
                                                const DevObstacle *__restrict__ obstacles,
@@ -34,59 +31,9 @@ __global__ void __launch_bounds__(256) k_grid(GridTable g, GridTable nxt, SimPar
     if (threadIdx.x == 0) s_abort = (*reinterpret_cast<volatile uint32_t *>(status) & kFatal) != 0;
     __syncthreads();
     if (s_abort) return;
-    const size_t gtid = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
-    uint32_t nblocks = min(*g.count, g.max_blocks);
-    constexpr int kM = (1 << BS) - 1;
-    const size_t nodes = static_cast<size_t>(nblocks) << (3 * BS);
-    float4 *next_pool = nxt.pool;
-    for (size_t node = gtid; node < nodes; node += stride) {
-        float4 mp = g.pool[node];
-        // the other pool receives the next P2G: zero every allocated block of it
-        if (next_pool) next_pool[node] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (mp.x <= 0.0f) {
-            g.pool[node] = make_float4(0.f, 0.f, 0.f, 0.f);
-            continue;
-        }
-        int4 c = g.coords[node >> (3 * BS)];
-        int l = static_cast<int>(node) & ((1 << (3 * BS)) - 1);
-        int cx = (c.x << BS) + (l >> (2 * BS)), cy = (c.y << BS) + ((l >> BS) & kM), cz = (c.z << BS) + (l & kM);
-        const SceneParams *const scn = sp.scenes + (MULTI ? (static_cast<uint32_t>(c.w) >> kSceneShift) : 0u);
-#define SCN(f) (MULTI ? scn->f : sp.s0.f)
-        const float h = SCN(h), dt = SCN(dt);
-        V3f vel = mk(mp.y / mp.x + SCN(gx) * dt, mp.z / mp.x + SCN(gy) * dt, mp.w / mp.x + SCN(gz) * dt);
-        V3f pos = mk(static_cast<float>(cx) * h, static_cast<float>(cy) * h, static_cast<float>(cz) * h);
-        if (SCN(has_bounds)) {
-            // walls by node index (thresholds from the f64 comparisons, see SceneParams)
-            const int ci[3] = {cx, cy, cz};
-            if (SCN(wall_mode) == 1) {
-                bool near = false;
-                for (int a = 0; a < 3; ++a) near = near || ci[a] <= SCN(wall_lo[a]) || ci[a] >= SCN(wall_hi[a]);
-                if (near) vel = mk(0, 0, 0);
-            } else {
-                for (int a = 0; a < 3; ++a) {
-                    const float va = comp(vel, a);
-                    if ((ci[a] <= SCN(wall_lo[a]) && va < 0.0f) || (ci[a] >= SCN(wall_hi[a]) && va > 0.0f))
-                        set_comp(vel, a, 0.0f);
-                }
-            }
-        }
-#undef SCN
-        for (int oi = 0; OBST && oi < sp.num_obstacles; ++oi) {
-            const DevObstacle &o = obstacles[oi];
-            if (!obstacle_may_contact(o, pos, h)) continue;
-            V3f nrm;
-            float d = obstacle_surface(o, planes, pos, nrm);
-            if (d <= h * (1.0f + 1e-5f)) {
-                V3f before = vel;
-                vel = contact_velocity(o, pos, vel, nrm);
-                if (sp.reactions)
-                    add_reaction(reactions, oi, mk(o.center[0], o.center[1], o.center[2]), pos - nrm * d,
-                                 (before - vel) * mp.x);
-            }
-        }
-        g.pool[node] = make_float4(vel.x, vel.y, vel.z, mp.x);
-    }
+    grid_nodes<MULTI, BS, OBST>(g, nxt.pool, sp, obstacles, planes, reactions,
+                                static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x,
+                                static_cast<size_t>(gridDim.x) * blockDim.x);
 }
 
 __global__ void k_clear_table(GridTable g) {
@@ -253,6 +200,22 @@ void launch_transfer(int mode, const ParticleSoA &P, int n, const DevClass *clas
     else if (sp.cpic) TMPM_VARIANT(kCpic);
     else if (sp.has_plastic || sp.num_obstacles > 0) TMPM_VARIANT(kPlainObst);
     else TMPM_VARIANT(kPlain);
+#undef TMPM_VARIANT
+}
+
+bool launch_small_segment(const ParticleSoA &P, int n, const DevClass *classes, const GridTable &cur,
+                          const GridTable &next, const SimParams &sp, const DevObstacle *obstacles,
+                          const float *planes, double *reactions, uint32_t *status, int *cache, int seg,
+                          uint32_t *arrived, cudaStream_t stream) {
+    if (n <= 0 || seg <= 0 || !arrived || sp.cpic) return false;
+    SimParams one = sp;
+    one.defer = nullptr;  // nothing is deferred: every chunk runs the general path
+#define TMPM_VARIANT(V)                                                                                            \
+    launch_segment_variant<V>(P, n, classes, cur, next, one, obstacles, planes, reactions, status, cache, seg, arrived, \
+                              stream)
+    if (sp.multi) return TMPM_VARIANT(kMulti);
+    if (sp.has_plastic || sp.num_obstacles > 0) return TMPM_VARIANT(kPlainObst);
+    return TMPM_VARIANT(kPlain);
 #undef TMPM_VARIANT
 }
 

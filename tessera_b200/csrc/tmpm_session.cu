@@ -422,7 +422,6 @@ struct TmpmSession {
     // update, transfer) with the last transfer G2P-only; the one-shot forces
     // act in the first substep and are cleared after it when `apply_force`.
     void launch_segment(const SimParams &sp, int from, bool resort, uint32_t seg, bool apply_force) {
-        const int bs = sp.block_shift;
         const int rows = resort ? from ^ 1 : from;
         if (resort) {
             ParticleSoA src = pbuf[from].view(force.ptr, std::max<size_t>(world.n, 1));
@@ -430,12 +429,25 @@ struct TmpmSession {
             SortBuffers sb = sort_buffers();
             launch_resort(src, dst, n_dev, n_dev, classes.ptr, sp, sb, stream);
         }
+        launch_steps(sp, rows, seg, apply_force);
+    }
+
+    // The table clear, P2G and substeps of a segment on row buffer `rows`: a
+    // small scene in one launch, otherwise kernel by kernel.
+    void launch_steps(const SimParams &sp, int rows, uint32_t seg, bool apply_force) {
+        const int bs = sp.block_shift;
         GridTable g[2];
         grid_views(g, bs);
         const ParticleSoA P = pbuf[rows].view(force.ptr, std::max<size_t>(world.n, 1));
         launch_clear_table(g[0], g[1], bs, stream);
         const SimParams sp0 = substep_params(sp, -1, false);
         open_defer_lists(sp0);
+        if (launch_small_segment(P, n_dev, classes.ptr, g[1], g[0], substep_params(sp, -1, apply_force),
+                                 dev_obstacles.ptr, dev_planes.ptr, reactions.ptr, status.ptr, cta_cache.ptr,
+                                 static_cast<int>(seg), sp0.defer ? sp0.defer + kBarrierWord : nullptr, stream)) {
+            if (apply_force) cudaMemsetAsync(force.ptr, 0, sizeof(float) * force.count, stream);
+            return;
+        }
         launch_transfer(kModeP2G, P, n_dev, classes.ptr, g[1], g[0], sp0, dev_obstacles.ptr, dev_planes.ptr,
                         reactions.ptr, status.ptr, cta_cache.ptr, stream);
         for (uint32_t k = 0; k < seg; ++k) {
@@ -592,6 +604,9 @@ struct TmpmSession {
                     tock(4);
                 }
                 if (tunable) tuner.begin(config, stream);
+                if (!kernel_ms) {
+                    launch_steps(sp, resort ? cur ^ 1 : cur, seg, apply_force);
+                } else {
                 GridTable g[2];
                 grid_views(g, bs);
                 const ParticleSoA P = pbuf[resort ? cur ^ 1 : cur].view(force.ptr, std::max<size_t>(world.n, 1));
@@ -616,6 +631,7 @@ struct TmpmSession {
                                     stream, &fj);
                     tock(last ? 3 : 2);
                     if (apply_force && k == 0) cudaMemsetAsync(force.ptr, 0, sizeof(float) * force.count, stream);
+                }
                 }
                 if (tunable) tuner.end(static_cast<double>(n_dev) * seg, stream);
             }

@@ -17,9 +17,10 @@
 // chunks the common path does not cover (see transfer_chunk).
 #pragma once
 
+#include <algorithm>
 #include <climits>
 
-#include "tmpm_device.cuh"
+#include "tmpm_grid.cuh"
 
 namespace tmpm {
 
@@ -407,7 +408,8 @@ __device__ __forceinline__ int record_tag(int step_index) { return 1 + (step_ind
 // 64 registers 24 / 28 bytes of spill stores / loads against 52 / 84 with the
 // fallbacks compiled in.
 template <int MODE, bool PLASTIC, int VARIANT, int THREADS, int BS, bool FAST>
-__device__ __forceinline__ void transfer_chunk(TMPM_TRANSFER_PARAMS, const int chunk) {
+__device__ __forceinline__ void transfer_chunk(TMPM_TRANSFER_PARAMS, const int chunk, const int step_index,
+                                               const int apply_force) {
     constexpr bool MULTI = VARIANT == kMulti;
     constexpr bool CPIC = VARIANT == kCpic;
     constexpr bool OBST = has_obstacles(VARIANT);
@@ -463,8 +465,8 @@ __device__ __forceinline__ void transfer_chunk(TMPM_TRANSFER_PARAMS, const int c
     if (MULTI && valid) {
         const int steps = scn->steps;
         const bool dead = (__ldcg(sp.scene_status + scene) & kStatusResident) != 0;
-        g2p_on = !dead && sp.step_index < steps;
-        p2g_on = !dead && sp.step_index + 1 < steps;
+        g2p_on = !dead && step_index < steps;
+        p2g_on = !dead && step_index + 1 < steps;
     }
     uint32_t *const resident_flag = MULTI ? sp.scene_status + scene : status;
     // grid namespace at the current positions (colour, and CPIC side masks when on)
@@ -500,7 +502,7 @@ __device__ __forceinline__ void transfer_chunk(TMPM_TRANSFER_PARAMS, const int c
         // The negative tag says that the P2G took the direct path: so does the
         // gather, without another box reduction.
         const int record = cc[0];
-        bool use_cache = record == record_tag(sp.step_index);
+        bool use_cache = record == record_tag(step_index);
         if constexpr (FAST) {
             if (!use_cache) return;  // on the no-record list (CTA-uniform)
         }
@@ -524,7 +526,7 @@ __device__ __forceinline__ void transfer_chunk(TMPM_TRANSFER_PARAMS, const int c
                 bx.nbt = cc[15];
                 bx.ok = 1;
                 tile_strides(bx.dim[1], bx.dim[2], bx.s1, bx.s2);
-            } else if (!FAST && record == -record_tag(sp.step_index)) {
+            } else if (!FAST && record == -record_tag(step_index)) {
                 bx.ok = 0;
                 bx.color = 0;
             } else if constexpr (!FAST) {
@@ -670,7 +672,7 @@ __device__ __forceinline__ void transfer_chunk(TMPM_TRANSFER_PARAMS, const int c
         V3f pos = x;
         if (updates) {
             // Particle update (gpu.wgsl:885-1003; world.rs:443-463).
-            if (sp.apply_force) {
+            if (apply_force) {
                 const size_t w = P.widx[i], fs = P.force_stride;
                 V3f f = mk(P.force[w], P.force[fs + w], P.force[2 * fs + w]);
                 vel = vel + mk(f.x / k.mass, f.y / k.mass, f.z / k.mass) * dt;  // force / mass * dt (gpu.wgsl:885)
@@ -956,7 +958,7 @@ __device__ __forceinline__ void transfer_chunk(TMPM_TRANSFER_PARAMS, const int c
             cc[kCacheHeader + t] = id;
         }
         if (threadIdx.x == 0) {
-            cc[0] = record_tag(sp.step_index + 1);
+            cc[0] = record_tag(step_index + 1);
             cc[1] = bx.blo[0];
             cc[2] = bx.blo[1];
             cc[3] = bx.blo[2];
@@ -991,8 +993,8 @@ __device__ __forceinline__ void transfer_chunk(TMPM_TRANSFER_PARAMS, const int c
         }
     } else {
         if (threadIdx.x == 0) {
-            cc[0] = -record_tag(sp.step_index + 1);
-            if (sp.defer) defer_push(sp, 2 + ((sp.step_index + 1) & 1), chunk);
+            cc[0] = -record_tag(step_index + 1);
+            if (sp.defer) defer_push(sp, 2 + ((step_index + 1) & 1), chunk);
         }
         if (active) {
             // Per-node global scatter, the stencil's blocks found or inserted
@@ -1023,13 +1025,13 @@ __device__ __forceinline__ void transfer_chunk(TMPM_TRANSFER_PARAMS, const int c
 // The general transfer: every chunk, one CTA each.
 template <int MODE, bool PLASTIC, int VARIANT, int THREADS, int MINB, int BS>
 __global__ void __launch_bounds__(THREADS, MINB) k_transfer(TMPM_TRANSFER_PARAMS) {
-    transfer_chunk<MODE, PLASTIC, VARIANT, THREADS, BS, false>(TMPM_TRANSFER_ARGS, blockIdx.x);
+    transfer_chunk<MODE, PLASTIC, VARIANT, THREADS, BS, false>(TMPM_TRANSFER_ARGS, blockIdx.x, sp.step_index, sp.apply_force);
 }
 
 // The fast fused transfer: every chunk with a record of this step.
 template <bool PLASTIC, int VARIANT, int THREADS, int MINB, int BS>
 __global__ void __launch_bounds__(THREADS, MINB) k_transfer_fast(TMPM_TRANSFER_PARAMS) {
-    transfer_chunk<kModeG2P2G, PLASTIC, VARIANT, THREADS, BS, true>(TMPM_TRANSFER_ARGS, blockIdx.x);
+    transfer_chunk<kModeG2P2G, PLASTIC, VARIANT, THREADS, BS, true>(TMPM_TRANSFER_ARGS, blockIdx.x, sp.step_index, sp.apply_force);
 }
 
 // The deferred chunks of a fast fused transfer through the general path, a
@@ -1050,19 +1052,92 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? TMPM_TRANSFER_MIN_BL
         for (uint32_t e = blockIdx.x; e < count; e += gridDim.x) {
             __syncthreads();  // the previous chunk's last reads of shared memory
             transfer_chunk<kModeG2P2G, PLASTIC, VARIANT, THREADS, BS, false>(
-                TMPM_TRANSFER_ARGS, static_cast<int>(lists[list * cap + e]));
+                TMPM_TRANSFER_ARGS, static_cast<int>(lists[list * cap + e]), sp.step_index, sp.apply_force);
         }
     } else {
         const uint32_t np = min(sp.defer[0], cap), nw = min(sp.defer[1], cap);
         for (uint32_t e = blockIdx.x; e < np + nw; e += gridDim.x) {
             __syncthreads();
             if (e < np)
-                transfer_chunk<kModeP2G, PLASTIC, VARIANT, THREADS, BS, false>(TMPM_TRANSFER_ARGS,
-                                                                               static_cast<int>(lists[e]));
+                transfer_chunk<kModeP2G, PLASTIC, VARIANT, THREADS, BS, false>(
+                    TMPM_TRANSFER_ARGS, static_cast<int>(lists[e]), sp.step_index, sp.apply_force);
             else
                 transfer_chunk<kModeG2P2G, PLASTIC, VARIANT, THREADS, BS, false>(
-                    TMPM_TRANSFER_ARGS, static_cast<int>(lists[cap + (e - np)]));
+                    TMPM_TRANSFER_ARGS, static_cast<int>(lists[cap + (e - np)]), sp.step_index, sp.apply_force);
         }
+    }
+}
+
+// Arrive at barrier number `target / gridDim.x` of a cooperative launch and
+// wait for every CTA.  The wait is bounded: on giving up it sets the timeout
+// bit and every CTA leaves (the same bit ends their waits).  Returns false
+// then.
+__device__ __forceinline__ bool grid_barrier(uint32_t *arrived, uint32_t target, uint32_t *status) {
+    __shared__ int s_ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        cuda::atomic_ref<uint32_t, cuda::thread_scope_device> a(*arrived);
+        __threadfence();
+        a.fetch_add(1u, cuda::memory_order_release);
+        int ok = 0;
+        for (int it = 0; it < kBarrierSpins; ++it) {
+            if (a.load(cuda::memory_order_acquire) >= target) {
+                ok = 1;
+                break;
+            }
+            if ((it & 1023) == 1023 && (*reinterpret_cast<volatile uint32_t *>(status) & kStatusTimeout)) break;
+        }
+        if (!ok) atomicOr(status, kStatusTimeout);
+        __threadfence();
+        s_ok = ok;
+    }
+    __syncthreads();
+    return s_ok != 0;
+}
+
+// A whole segment of a small scene (or batch) in one cooperative launch: the
+// opening P2G, then `seg` substeps of grid update and fused transfer, the last
+// one G2P-only, with a grid-wide barrier between phases.
+//
+// At these sizes a substep's kernels are each a partial wave and the time goes
+// into launches, the fork and join of the deferred chunks and the tails of
+// dependent kernels; every phase here starts one barrier after the last.  All
+// chunks take the general path (there are registers for it at two CTAs of 256
+// particles an SM), so nothing is deferred.  Chunk c belongs to CTA c %
+// gridDim.x in every phase: particle rows and the chunk's record are only read
+// by the SM that wrote them; grid data is read through L2.
+template <bool PLASTIC, int VARIANT, int THREADS, int BS>
+__global__ void __launch_bounds__(THREADS, kSegmentThreads / THREADS)
+    k_segment(TMPM_TRANSFER_PARAMS, int seg, uint32_t *arrived) {
+    const int chunks = (n + THREADS - 1) / THREADS;
+    uint32_t target = 0;
+    for (int c = blockIdx.x; c < chunks; c += gridDim.x) {
+        __syncthreads();
+        transfer_chunk<kModeP2G, PLASTIC, VARIANT, THREADS, BS, false>(TMPM_TRANSFER_ARGS, c, -1, 0);
+    }
+    GridTable a = next, b = cur;  // one table, two pools: `a` holds the nodes of the substep at hand
+    for (int k = 0; k < seg; ++k) {
+        target += gridDim.x;
+        if (!grid_barrier(arrived, target, status)) return;
+        if (!(*reinterpret_cast<volatile uint32_t *>(status) & kFatal))
+            grid_nodes<VARIANT == kMulti, BS, has_obstacles(VARIANT)>(
+                a, b.pool, sp, obstacles, planes, reactions, static_cast<size_t>(blockIdx.x) * THREADS + threadIdx.x,
+                static_cast<size_t>(gridDim.x) * THREADS);
+        target += gridDim.x;
+        if (!grid_barrier(arrived, target, status)) return;
+        const int force = k == 0 ? sp.apply_force : 0;
+        for (int c = blockIdx.x; c < chunks; c += gridDim.x) {
+            __syncthreads();
+            if (k + 1 < seg)
+                transfer_chunk<kModeG2P2G, PLASTIC, VARIANT, THREADS, BS, false>(
+                    P, n, classes, a, b, sp, obstacles, planes, reactions, status, cache, c, k, force);
+            else
+                transfer_chunk<kModeG2P, PLASTIC, VARIANT, THREADS, BS, false>(
+                    P, n, classes, a, b, sp, obstacles, planes, reactions, status, cache, c, k, force);
+        }
+        float4 *const pool = a.pool;
+        a.pool = b.pool;
+        b.pool = pool;
     }
 }
 #undef TMPM_TRANSFER_ARGS
@@ -1150,6 +1225,49 @@ void launch_transfer_variant(int mode, const ParticleSoA &P, int n, const DevCla
 }
 
 namespace {
+// Launch k_segment if every chunk has a CTA resident at once.
+template <bool PL, int V, int T, int BS>
+bool try_segment(const ParticleSoA &P, int n, const DevClass *classes, const GridTable &cur, const GridTable &next,
+                 const SimParams &sp, const DevObstacle *obstacles, const float *planes, double *reactions,
+                 uint32_t *status, int *cache, int seg, uint32_t *arrived, cudaStream_t stream) {
+    const int chunks = (n + T - 1) / T;
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_segment<PL, V, T, BS>, T, 0) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    const int room = per_sm * device_sm_count();
+    if (room <= 0 || chunks > kSegmentChunksPerCta * room) return false;
+    void *args[] = {const_cast<ParticleSoA *>(&P), &n, &classes, const_cast<GridTable *>(&cur),
+                    const_cast<GridTable *>(&next), const_cast<SimParams *>(&sp), &obstacles, &planes, &reactions,
+                    &status, &cache, &seg, &arrived};
+    if (cudaLaunchCooperativeKernel(k_segment<PL, V, T, BS>, dim3(std::min(chunks, room)), dim3(T), args, 0, stream) ==
+        cudaSuccess)
+        return true;
+    cudaGetLastError();
+    return false;
+}
+}  // namespace
+
+template <int V>
+bool launch_segment_variant(const ParticleSoA &P, int n, const DevClass *classes, const GridTable &cur,
+                            const GridTable &next, const SimParams &sp, const DevObstacle *obstacles,
+                            const float *planes, double *reactions, uint32_t *status, int *cache, int seg,
+                            uint32_t *arrived, cudaStream_t stream) {
+#define TMPM_SEGMENT(PL, T, BS) \
+    try_segment<PL, V, T, BS>(P, n, classes, cur, next, sp, obstacles, planes, reactions, status, cache, seg, arrived, stream)
+    if (sp.has_plastic) {
+        if constexpr (V == kPlainObst) return TMPM_SEGMENT(true, 256, kBlockShift);
+        return false;
+    }
+    const bool narrow = kLaunchShapes[sp.shape].threads == 128;
+    if (sp.block_shift == kBigBlockShift)
+        return narrow ? TMPM_SEGMENT(false, 128, kBigBlockShift) : TMPM_SEGMENT(false, 256, kBigBlockShift);
+    return narrow ? TMPM_SEGMENT(false, 128, kBlockShift) : TMPM_SEGMENT(false, 256, kBlockShift);
+#undef TMPM_SEGMENT
+}
+
+namespace {
 template <int V, int T, int B, int BS>
 void touch_shape() {
     cudaFuncAttributes a;
@@ -1159,6 +1277,7 @@ void touch_shape() {
     cudaFuncGetAttributes(&a, k_transfer<kModeP2G, false, V, T, B, BS>);
     cudaFuncGetAttributes(&a, k_transfer<kModeG2P2G, false, V, T, B, BS>);
     cudaFuncGetAttributes(&a, k_transfer<kModeG2P, false, V, T, B, BS>);
+    cudaFuncGetAttributes(&a, k_segment<false, V, T, BS>);
 }
 }  // namespace
 
@@ -1178,5 +1297,10 @@ void preload_transfer_variant() {
                                                   const GridTable &, const SimParams &, const DevObstacle *, \
                                                   const float *, double *, uint32_t *, int *, cudaStream_t, \
                                                   const ForkJoin *);
+
+#define TMPM_SEGMENT_VARIANT(V)                                                                                      \
+    template bool launch_segment_variant<V>(const ParticleSoA &, int, const DevClass *, const GridTable &,           \
+                                            const GridTable &, const SimParams &, const DevObstacle *, const float *, \
+                                            double *, uint32_t *, int *, int, uint32_t *, cudaStream_t);
 
 }  // namespace tmpm

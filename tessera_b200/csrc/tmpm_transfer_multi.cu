@@ -3,5 +3,6 @@
 
 namespace tmpm {
 TMPM_TRANSFER_VARIANT(kMulti)
+TMPM_SEGMENT_VARIANT(kMulti)
 template void preload_transfer_variant<kMulti>();
 }  // namespace tmpm

@@ -3,5 +3,6 @@
 
 namespace tmpm {
 TMPM_TRANSFER_VARIANT(kPlainObst)
+TMPM_SEGMENT_VARIANT(kPlainObst)
 template void preload_transfer_variant<kPlainObst>();
 }  // namespace tmpm

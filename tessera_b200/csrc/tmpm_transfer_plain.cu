@@ -3,5 +3,6 @@
 
 namespace tmpm {
 TMPM_TRANSFER_VARIANT(kPlain)
+TMPM_SEGMENT_VARIANT(kPlain)
 template void preload_transfer_variant<kPlain>();
 }  // namespace tmpm
