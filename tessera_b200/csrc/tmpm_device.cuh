@@ -136,7 +136,8 @@ __device__ __forceinline__ M3f scaled_stress(const DevClass &k, const M3f &F, co
     } else if (k.kind == kMatFluid) {
         float bulk = k.p0, gamma = k.p1, visc = k.p2, tensile = k.p3;
         float sj = fmaxf(J, 1e-6f);
-        float pressure = sj <= 1.0f ? bulk * (powf(sj, -gamma) - 1.0f) : -bulk * tensile * (sj - 1.0f);
+        // bulk (J^-gamma - 1) without the cancellation of 1 near J = 1
+        float pressure = sj <= 1.0f ? bulk * expm1f(-gamma * logf(sj)) : -bulk * tensile * (sj - 1.0f);
         M3f sr = scale(add(Cm, transpose(Cm)), 0.5f);
         float tr3 = (sr.c0.x + sr.c1.y + sr.c2.z) * (1.0f / 3.0f);
         float diag = -2.0f * visc * sj * tr3 - pressure * sj;
@@ -726,6 +727,33 @@ __device__ __forceinline__ void red_add_v4(float4 *addr, float4 v) {
     asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(addr), "f"(v.x), "f"(v.y), "f"(v.z),
                  "f"(v.w)
                  : "memory");
+}
+
+// Arrive at barrier number `target / gridDim.x` of a cooperative launch and
+// wait for every CTA.  The wait is bounded: on giving up it sets the timeout
+// bit and every CTA leaves (the same bit ends their waits).  Returns false
+// then.
+__device__ __forceinline__ bool grid_barrier(uint32_t *arrived, uint32_t target, uint32_t *status) {
+    __shared__ int s_ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        cuda::atomic_ref<uint32_t, cuda::thread_scope_device> a(*arrived);
+        __threadfence();
+        a.fetch_add(1u, cuda::memory_order_release);
+        int ok = 0;
+        for (int it = 0; it < kBarrierSpins; ++it) {
+            if (a.load(cuda::memory_order_acquire) >= target) {
+                ok = 1;
+                break;
+            }
+            if ((it & 1023) == 1023 && (*reinterpret_cast<volatile uint32_t *>(status) & kStatusTimeout)) break;
+        }
+        if (!ok) atomicOr(status, kStatusTimeout);
+        __threadfence();
+        s_ok = ok;
+    }
+    __syncthreads();
+    return s_ok != 0;
 }
 
 }  // namespace tmpm

@@ -1176,6 +1176,7 @@ TmpmStatus tmpm_debug_p2g(TmpmSession *s, int32_t *cells_out, float *mm_out, siz
     if (s->n_dev == 0) return TMPM_OK;
     cudaSetDevice(s->device);
     SimParams sp = s->sim_params(s->substep_dt, true);
+    sp.step_index = -1;  // a segment's opening P2G: every F is read whole
     GridTable gv[2];
     s->grid_views(gv, kBlockShift);
     GridTable g0 = gv[0], g1 = gv[1];
