@@ -297,7 +297,7 @@ TmpmStatus tmpm_step_cfl_with_reactions(TmpmSession *session, double dt,
  * session's re-sort uses.  `stream` is a cudaStream_t (NULL =
  * the default stream); the call is asynchronous on it.
  * It allocates nothing: its scratch is a fixed array inside the library
- * (4,260,864 bytes, held on every device that loads the library until exit),
+ * (4,980,736 bytes, held on every device that loads the library until exit),
  * so `count` is limited to 262,144; larger counts return TMPM_ERR_CAPACITY
  * with the reason in tmpm_last_error().  Set-up: a call made outside a stream
  * capture looks up the scratch address in the current context; a call made

@@ -340,10 +340,9 @@ struct TmpmBatch {
             ++epoch;
         }
         if (sort_keys[0].count < cap) {
-            const size_t tiles = (cap + 4095) / 4096;
             for (int b = 0; b < 2; ++b)
                 if ((e = sort_keys[b].alloc(cap)) || (e = sort_vals[b].alloc(cap))) return cuda_fail(e, "cudaMalloc sort");
-            if ((e = sort_hist.alloc(256 * tiles)) || (e = sort_totals.alloc(256))) return cuda_fail(e, "cudaMalloc sort");
+            if ((e = sort_hist.alloc(sort_hist_words(cap))) || (e = sort_totals.alloc(256))) return cuda_fail(e, "cudaMalloc sort");
             ++epoch;
         }
         return TMPM_OK;

@@ -664,6 +664,26 @@ __device__ __forceinline__ uint32_t morton_block(int bx, int by, int bz, uint32_
            (spread10(static_cast<uint32_t>(by) & 0x7Fu) << 1) | spread10(static_cast<uint32_t>(bz) & 0x7Fu);
 }
 
+// Sort key of position i (BinSource); `cells`, when given, gets its base cell.
+__device__ __forceinline__ uint32_t bin_key(const BinSource &s, int i, int32_t *cells = nullptr) {
+    float inv_h = s.inv_h;
+    uint32_t scene = 0;
+    if (s.scenes) {
+        scene = s.classes[s.cls[i] & kClassMask].color >> kSceneShift;
+        if (!s.scenes[scene].live) return kDeadKey;  // removed scene: sorts after every live particle
+        inv_h = s.scenes[scene].inv_h;
+    }
+    const int b0 = base_cell(s.x[i], inv_h), b1 = base_cell(s.x[s.cap + i], inv_h),
+              b2 = base_cell(s.x[2 * s.cap + i], inv_h);
+    if (cells) {
+        cells[3 * i] = b0;
+        cells[3 * i + 1] = b1;
+        cells[3 * i + 2] = b2;
+    }
+    const uint32_t block = morton_block(b0 >> kBlockShift, b1 >> kBlockShift, b2 >> kBlockShift, scene);
+    return s.scenes ? block : (block << 6) | cell_in_block(b0, b1, b2);
+}
+
 // Find the block id of `key`, allocating the block if absent.  Ids grow from
 // zero after each table clear and both node pools are zeroed with it, so a
 // new block's nodes are zero already (the grid update zeroes the blocks in use

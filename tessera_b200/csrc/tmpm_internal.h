@@ -233,7 +233,7 @@ struct ParticleSoA {
 struct SortBuffers {
     uint32_t *keys[2];
     uint32_t *vals[2];
-    uint32_t *hist;    // 256 * tiles
+    uint32_t *hist;    // sort_hist_words(cap)
     uint32_t *totals;  // 256
     size_t cap;
 };
@@ -326,11 +326,23 @@ void launch_clear_table(const GridTable &g, const GridTable &other, int block_sh
 // first `keep` particles are gathered.
 void launch_resort(ParticleSoA &src, ParticleSoA &dst, int n, int keep, const DevClass *classes, const SimParams &sp,
                    SortBuffers &sb, cudaStream_t stream);
-void launch_bin_keys(const ParticleSoA &P, int n, const DevClass *classes, const SimParams &sp, int32_t *cells,
-                     uint32_t *keys, cudaStream_t stream);
-// Morton block keys (and identity values) of `n` positions stored component-major with `stride`.
-void launch_bin_keys_values(const float *x, size_t stride, int n, float inv_h, uint32_t *keys, uint32_t *vals,
-                            cudaStream_t stream);
+// Where sort keys come from: `n` positions stored component-major with stride
+// `cap`.  Single scene (`scenes` null): the block's 21-bit Morton code followed by
+// the cell's 6-bit Morton code inside the block, so particles of one cell are
+// contiguous after the sort.  With a scene table (multi-scene batch): scene << 21
+// | block Morton, the scene from the particle's class and its cell width from the
+// table.
+struct BinSource {
+    const float *x;
+    size_t cap;
+    int n;
+    float inv_h;
+    const uint32_t *cls;
+    const DevClass *classes;
+    const SceneParams *scenes;
+};
+// Base cells (optional), keys and identity values (optional).
+void launch_bin_keys(const BinSource &src, int32_t *cells, uint32_t *keys, uint32_t *vals, cudaStream_t stream);
 void launch_dump_grid(const GridTable &g, int32_t *cells, float4 *values, uint32_t *count, uint32_t capacity,
                       int block_shift, cudaStream_t stream);
 void launch_snapshot(const ParticleSoA &P, int n, const DevClass *classes, float4 *out, cudaStream_t stream);
@@ -348,5 +360,13 @@ void set_last_error(const std::string &msg);
 // Radix sort (tmpm_sort.cu): stable sort of (key, value) pairs by `bits` low key
 // bits, 8 bits per pass.  Returns r: the result is in sb.keys[r] / sb.vals[r].
 int radix_sort_pairs(SortBuffers &sb, int n, int bits, cudaStream_t stream);
+// Keys of `src` and the stable sort of (key, index) by `bits` low key bits.
+// Without `vals_out` the result is in sb.keys[r] / sb.vals[r], r returned;
+// with it, there (`keys_out` may be null).
+constexpr size_t kSmallSort = size_t(1) << 18;  // up to here the sort is four kernels
+int bin_and_sort(const BinSource &src, SortBuffers &sb, int bits, uint32_t *keys_out, uint32_t *vals_out,
+                 cudaStream_t stream);
+// Words of SortBuffers::hist for sorts of up to `cap` keys.
+size_t sort_hist_words(size_t cap);
 
 }  // namespace tmpm

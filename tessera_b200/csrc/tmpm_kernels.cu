@@ -46,34 +46,10 @@ __global__ void k_clear_table(GridTable g) {
     if (gtid == 0) *g.count = 0;
 }
 
-// Sort key of each particle.  Single scene: the block's 21-bit Morton code
-// followed by the cell's 6-bit Morton code inside the block, so particles of
-// one cell are contiguous after the sort.  With a scene table (multi-scene
-// batch): scene << 21 | block Morton, the scene from the particle's class and
-// its cell width from the table.
-__global__ void k_bin_keys(const float *x, size_t cap, int n, float inv_h, const uint32_t *__restrict__ cls,
-                           const DevClass *__restrict__ classes, const SceneParams *__restrict__ scenes,
-                           int32_t *cells, uint32_t *keys, uint32_t *vals) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    uint32_t scene = 0;
-    if (scenes) {
-        scene = classes[cls[i] & kClassMask].color >> kSceneShift;
-        if (!scenes[scene].live) {  // removed scene: sorts after every live particle
-            keys[i] = kDeadKey;
-            if (vals) vals[i] = static_cast<uint32_t>(i);
-            return;
-        }
-        inv_h = scenes[scene].inv_h;
-    }
-    int b0 = base_cell(x[i], inv_h), b1 = base_cell(x[cap + i], inv_h), b2 = base_cell(x[2 * cap + i], inv_h);
-    if (cells) {
-        cells[3 * i] = b0;
-        cells[3 * i + 1] = b1;
-        cells[3 * i + 2] = b2;
-    }
-    const uint32_t block = morton_block(b0 >> kBlockShift, b1 >> kBlockShift, b2 >> kBlockShift, scene);
-    keys[i] = scenes ? block : (block << 6) | cell_in_block(b0, b1, b2);
+__global__ void k_bin_keys(BinSource src, int32_t *cells, uint32_t *keys, uint32_t *vals) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= src.n) return;
+    keys[i] = bin_key(src, i, cells);
     if (vals) vals[i] = static_cast<uint32_t>(i);
 }
 
@@ -258,26 +234,16 @@ void launch_clear_table(const GridTable &g, const GridTable &other, int block_sh
     if (other.pool != g.pool) cudaMemsetAsync(other.pool, 0, bytes, stream);
 }
 
-void launch_bin_keys(const ParticleSoA &P, int n, const DevClass *classes, const SimParams &sp, int32_t *cells,
-                     uint32_t *keys, cudaStream_t stream) {
-    if (n <= 0) return;
-    k_bin_keys<<<(n + 255) / 256, 256, 0, stream>>>(P.x, P.cap, n, sp.s0.inv_h, P.cls, classes,
-                                                    sp.multi ? sp.scenes : nullptr, cells, keys, nullptr);
-}
-
-void launch_bin_keys_values(const float *x, size_t stride, int n, float inv_h, uint32_t *keys, uint32_t *vals,
-                            cudaStream_t stream) {
-    if (n <= 0) return;
-    k_bin_keys<<<(n + 255) / 256, 256, 0, stream>>>(x, stride, n, inv_h, nullptr, nullptr, nullptr, nullptr, keys,
-                                                    vals);
+void launch_bin_keys(const BinSource &src, int32_t *cells, uint32_t *keys, uint32_t *vals, cudaStream_t stream) {
+    if (src.n <= 0) return;
+    k_bin_keys<<<(src.n + 255) / 256, 256, 0, stream>>>(src, cells, keys, vals);
 }
 
 void launch_resort(ParticleSoA &src, ParticleSoA &dst, int n, int keep, const DevClass *classes, const SimParams &sp,
                    SortBuffers &sb, cudaStream_t stream) {
     if (n <= 0) return;
-    k_bin_keys<<<(n + 255) / 256, 256, 0, stream>>>(src.x, src.cap, n, sp.s0.inv_h, src.cls, classes,
-                                                    sp.multi ? sp.scenes : nullptr, nullptr, sb.keys[0], sb.vals[0]);
-    const int r = radix_sort_pairs(sb, n, sp.multi ? kSortBitsBatch : kSortBitsScene, stream);
+    const BinSource bins{src.x, src.cap, n, sp.s0.inv_h, src.cls, classes, sp.multi ? sp.scenes : nullptr};
+    const int r = bin_and_sort(bins, sb, sp.multi ? kSortBitsBatch : kSortBitsScene, nullptr, nullptr, stream);
     const int interleave = sp.multi ? 0 : kLaunchShapes[sp.shape].threads;
     if (keep > 0) k_gather<<<(keep + 255) / 256, 256, 0, stream>>>(src, dst, sb.vals[r], keep, interleave);
 }

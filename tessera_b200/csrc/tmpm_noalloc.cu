@@ -22,10 +22,11 @@
 namespace {
 
 constexpr size_t kNoAllocMaxParticles = size_t(1) << 18;  // 262,144 particles per call
-constexpr size_t kNoAllocTiles = (kNoAllocMaxParticles + 4095) / 4096;
-// keys[2][max] | vals[2][max] | hist[256][tiles] | totals[256], 32-bit words:
-// 4 * 2^18 + 256 * 64 + 256 = 1,065,216 words = 4,260,864 bytes
-constexpr size_t kNoAllocWords = 4 * kNoAllocMaxParticles + 256 * kNoAllocTiles + 256;
+static_assert(kNoAllocMaxParticles <= tmpm::kSmallSort, "the scratch holds the small sort's histograms");
+constexpr size_t kNoAllocTiles = (kNoAllocMaxParticles + 2047) / 2048;
+// keys[2][max] | vals[2][max] | hist[3][tiles][512], 32-bit words:
+// 4 * 2^18 + 3 * 128 * 512 = 1,245,184 words = 4,980,736 bytes
+constexpr size_t kNoAllocWords = 4 * kNoAllocMaxParticles + 3 * kNoAllocTiles * 512;
 
 // Device-resident scratch shared by every call on a device.  Host code must
 // never hand this symbol itself to a kernel: on the host it is only a
@@ -68,6 +69,17 @@ CUcontext current_context() {
     CUcontext ctx = nullptr;
     if (!fn || fn(&ctx) != CUDA_SUCCESS) return nullptr;
     return ctx;
+}
+
+// Whether a kernel may write 32-bit words at `p`: device memory, aligned.
+bool device_words(const uint32_t *p) {
+    cudaPointerAttributes a{};
+    if (reinterpret_cast<uintptr_t>(p) % sizeof(uint32_t) != 0) return false;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeDevice;
 }
 
 }  // namespace
@@ -129,16 +141,20 @@ extern "C" TmpmStatus tmpm_sort_by_block_noalloc(const float *positions, size_t 
     sb.vals[0] = base + 2 * kNoAllocMaxParticles;
     sb.vals[1] = base + 3 * kNoAllocMaxParticles;
     sb.hist = base + 4 * kNoAllocMaxParticles;
-    sb.totals = sb.hist + 256 * kNoAllocTiles;
     sb.cap = kNoAllocMaxParticles;
     // Every scratch word this call reads is written earlier in the same call
-    // (keys and values by the binning kernel, histograms and totals by each
-    // radix pass), so nothing has to start at zero.
+    // (keys and values by the kernel before the one that reads them, histograms
+    // by the key kernel), so nothing has to start at zero.
     const int n = static_cast<int>(count);
-    tmpm::launch_bin_keys_values(positions, stride, n, 1.0f / h32, sb.keys[0], sb.vals[0], s);
-    const int r = tmpm::radix_sort_pairs(sb, n, tmpm::kSortBitsScene, s);
+    const tmpm::BinSource src{positions, stride, n, 1.0f / h32, nullptr, nullptr, nullptr};
+    // The last pass writes device buffers itself; anything else (a buffer that
+    // only a copy can reach, or one not aligned to its words) gets a copy.
+    const bool direct = device_words(order_out) && (!keys_out || device_words(keys_out));
+    const int r = tmpm::bin_and_sort(src, sb, tmpm::kSortBitsScene, direct ? keys_out : nullptr,
+                                     direct ? order_out : nullptr, s);
     e = cudaGetLastError();  // launch errors of the binning and radix kernels
     if (e != cudaSuccess) return noalloc_fail(TMPM_ERR_DEVICE, std::string("launch: ") + cudaGetErrorString(e));
+    if (direct) return TMPM_OK;
     e = cudaMemcpyAsync(order_out, sb.vals[r], sizeof(uint32_t) * count, cudaMemcpyDeviceToDevice, s);
     if (e != cudaSuccess)
         return noalloc_fail(TMPM_ERR_DEVICE, std::string("copy of the order: ") + cudaGetErrorString(e));

@@ -328,12 +328,11 @@ struct TmpmSession {
             if (grids[g].max_blocks != plan.blocks || grids[g].pool_nodes != plan.nodes)
                 if ((e = grids[g].alloc(static_cast<uint32_t>(plan.blocks), plan.nodes))) return cuda_fail(e, "cudaMalloc grid");
         size_t sort_cap = pbuf[0].cap;
-        size_t tiles = (sort_cap + 4095) / 4096;
         if (sort_keys[0].count < sort_cap) {
             for (int b = 0; b < 2; ++b)
                 if ((e = sort_keys[b].alloc(sort_cap)) || (e = sort_vals[b].alloc(sort_cap)))
                     return cuda_fail(e, "cudaMalloc sort");
-            if ((e = sort_hist.alloc(256 * tiles)) || (e = sort_totals.alloc(256))) return cuda_fail(e, "cudaMalloc sort");
+            if ((e = sort_hist.alloc(sort_hist_words(sort_cap))) || (e = sort_totals.alloc(256))) return cuda_fail(e, "cudaMalloc sort");
         }
         if ((e = classes.alloc(std::max<size_t>(cls_table.size(), 1)))) return cuda_fail(e, "cudaMalloc classes");
         if ((e = dev_obstacles.alloc(std::max<size_t>(dobs.size(), 1)))) return cuda_fail(e, "cudaMalloc obstacles");
@@ -1161,7 +1160,8 @@ TmpmStatus tmpm_debug_binning(TmpmSession *s, uint32_t *world_index_out, int32_t
     if ((e = cells.alloc(3 * static_cast<size_t>(n))) || (e = keys.alloc(n))) return s->cuda_fail(e, "cudaMalloc");
     SimParams sp = s->sim_params(s->substep_dt, true);
     ParticleSoA P = s->soa();
-    launch_bin_keys(P, n, s->classes.ptr, sp, cells.ptr, keys.ptr, s->stream);
+    launch_bin_keys(BinSource{P.x, P.cap, n, sp.s0.inv_h, nullptr, nullptr, nullptr}, cells.ptr, keys.ptr, nullptr,
+                    s->stream);
     if (world_index_out) cudaMemcpyAsync(world_index_out, P.widx, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, s->stream);
     if (base_cell_out) cudaMemcpyAsync(base_cell_out, cells.ptr, sizeof(int32_t) * 3 * n, cudaMemcpyDeviceToHost, s->stream);
     if (key_out) cudaMemcpyAsync(key_out, keys.ptr, sizeof(uint32_t) * n, cudaMemcpyDeviceToHost, s->stream);
