@@ -632,6 +632,11 @@ struct TmpmBatch {
         g[1] = g[0];
         g[1].pool = grids[1].pool.ptr;
         const int n = static_cast<int>(n_live);
+        SimParams sp0 = sp;
+        sp0.step_index = -1;
+        if (launch_small_segment(dst, n, dclasses.ptr, g[1], g[0], sp0, nullptr, nullptr, nullptr, status.ptr,
+                                 cta_cache.ptr, static_cast<int>(steps), stream))
+            return;
         launch_clear_table(g[0], g[1], bs, stream);
         // the fused transfer's deferred-chunk lists (as in a session): emptied
         // before the opening P2G, then by each grid update for its transfer
@@ -640,12 +645,8 @@ struct TmpmBatch {
                                             ? (defer.count - kDeferHeader) / 4
                                             : 0);
         if (sp.defer) cudaMemsetAsync(sp.defer, 0, sizeof(uint32_t) * kDeferHeader, stream);
-        SimParams sp0 = sp;
+        sp0 = sp;
         sp0.step_index = -1;
-        if (launch_small_segment(dst, n, dclasses.ptr, g[1], g[0], sp0, nullptr, nullptr, nullptr, status.ptr,
-                                 cta_cache.ptr, static_cast<int>(steps), sp.defer ? sp.defer + kBarrierWord : nullptr,
-                                 stream))
-            return;
         launch_transfer(kModeP2G, dst, n, dclasses.ptr, g[1], g[0], sp0, nullptr, nullptr, nullptr, status.ptr,
                         cta_cache.ptr, stream);
         for (uint32_t s = 0; s < steps; ++s) {

@@ -755,21 +755,23 @@ __device__ __forceinline__ void red_add_v4(float4 *addr, float4 v) {
 // then.
 __device__ __forceinline__ bool grid_barrier(uint32_t *arrived, uint32_t target, uint32_t *status) {
     __shared__ int s_ok;
+    // The release covers the whole CTA's writes (ordered before it by the block
+    // barrier), the acquire its later reads; no return value and no fence of its
+    // own: 1.6 -> 0.9 us for two CTAs against fetch_add between two fences.
     __syncthreads();
     if (threadIdx.x == 0) {
-        cuda::atomic_ref<uint32_t, cuda::thread_scope_device> a(*arrived);
-        __threadfence();
-        a.fetch_add(1u, cuda::memory_order_release);
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(arrived) : "memory");
         int ok = 0;
         for (int it = 0; it < kBarrierSpins; ++it) {
-            if (a.load(cuda::memory_order_acquire) >= target) {
+            uint32_t seen;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(arrived) : "memory");
+            if (seen >= target) {
                 ok = 1;
                 break;
             }
             if ((it & 1023) == 1023 && (*reinterpret_cast<volatile uint32_t *>(status) & kStatusTimeout)) break;
         }
         if (!ok) atomicOr(status, kStatusTimeout);
-        __threadfence();
         s_ok = ok;
     }
     __syncthreads();

@@ -719,9 +719,11 @@ struct GridBuffers {
         uint32_t cap = 1024;
         while (cap < 2u * blocks) cap <<= 1;
         cudaError_t e;
-        if ((e = keys.alloc(cap)) || (e = vals.alloc(cap)) || (e = count.alloc(1)) || (e = pool.alloc(nodes)) ||
+        if ((e = keys.alloc(cap)) || (e = vals.alloc(cap)) || (e = count.alloc(kTableWords)) || (e = pool.alloc(nodes)) ||
             (e = coords.alloc(blocks)))
             return e;
+        const uint32_t words[kTableWords] = {0, ~0u, 0, 0};
+        if ((e = cudaMemcpy(count.ptr, words, sizeof words, cudaMemcpyHostToDevice))) return e;
         capacity = cap;
         max_blocks = blocks;
         pool_nodes = nodes;
@@ -735,6 +737,7 @@ struct GridBuffers {
         g.pool = pool.ptr;
         g.coords = coords.ptr;
         g.mask = capacity - 1;
+        g.pool_nodes = pool_nodes;
         g.max_blocks = static_cast<uint32_t>(std::min<size_t>(max_blocks, pool_nodes >> (3 * block_shift)));
         return g;
     }

@@ -65,16 +65,14 @@ constexpr int kNumLaunchShapes = 3;
 constexpr int kNumLaunchConfigs = 2 * kNumLaunchShapes;
 constexpr int config_shape(int c) { return c % kNumLaunchShapes; }
 constexpr int config_block_shift(int c) { return c < kNumLaunchShapes ? kBlockShift : kBigBlockShift; }
-// A whole-segment kernel runs this many threads an SM (128 registers each, which
-// the general path needs) and at most so many chunks per CTA.
+// A whole-segment kernel runs up to this many threads an SM (128 registers each,
+// which the general path needs) and takes a scene whose chunks are all resident
+// at once: 75,776 particles on 148 SMs.  Above, kernel by kernel is faster
+// (85,184 particles: 30.1 us a substep against 34.1 with two chunks a CTA).
 constexpr int kSegmentThreads = 512;
-#ifndef TMPM_SEGMENT_CHUNKS
-#define TMPM_SEGMENT_CHUNKS 1
-#endif
-constexpr int kSegmentChunksPerCta = TMPM_SEGMENT_CHUNKS;
 constexpr int kBarrierSpins = 1 << 24;  // bounded wait at its barriers (a few seconds)
 constexpr int kMinTransferThreads = 128;  // per-CTA records are sized for the smallest shape
-constexpr int kCacheStride = 144;      // per-CTA record: 16-int box header + up to 128 block ids
+constexpr int kCacheStride = 272;      // per-CTA record: 16-int box header + up to 256 block ids
 
 constexpr uint32_t kFixedBit = 0x80000000u;
 constexpr uint32_t kClassMask = 0x7FFFFFFFu;
@@ -162,12 +160,17 @@ struct RigidParams {
 struct GridTable {
     unsigned long long *keys;  // [capacity]
     uint32_t *vals;            // [capacity]
-    uint32_t *count;           // allocated blocks
+    uint32_t *count;           // kTableWords words: allocated blocks, then the words below
     float4 *pool;              // [max_blocks * 64]
     int4 *coords;              // [max_blocks]: bx, by, bz, colour
     uint32_t mask;             // capacity - 1
     uint32_t max_blocks;
+    size_t pool_nodes;         // float4 nodes of the pool
 };
+// Words after a table's block count: how many leading nodes of the two pools may
+// be non-zero (a whole-segment kernel clears those; anything else leaves ~0),
+// and the arrivals and departures of its barriers.
+constexpr int kDirtyWord = 1, kBarrierWord = 2, kExitWord = 3, kTableWords = 4;
 
 // Grid namespace of a particle class in a multi-scene batch: scene << kSceneShift | colour.
 constexpr int kSceneShift = 8;
@@ -208,10 +211,8 @@ static_assert(sizeof(SimParams) == sizeof(SceneParams) + 3 * sizeof(void *) + 12
 
 // Deferred-chunk lists of the fast fused transfer, in one device buffer of
 // kDeferHeader + 4 * cap words: counts [0] P2G-only, [1] whole chunk,
-// [2 + p] no record for a launch of step parity p, [kBarrierWord] arrivals at
-// a whole-segment kernel's barriers; then the lists in that order (cap entries
-// each).
-constexpr int kBarrierWord = 4;
+// [2 + p] no record for a launch of step parity p; then the lists in that
+// order (cap entries each).
 constexpr int kDeferHeader = 8;
 inline size_t defer_words(size_t cap) { return kDeferHeader + 4 * cap; }
 static_assert(sizeof(SceneParams) == 30 * sizeof(float), "SceneParams must have no padding bytes");
@@ -277,7 +278,7 @@ template <int V>
 bool launch_segment_variant(const ParticleSoA &P, int n, const DevClass *classes, const GridTable &cur,
                             const GridTable &next, const SimParams &sp, const DevObstacle *obstacles,
                             const float *planes, double *reactions, uint32_t *status, int *cache, int seg,
-                            uint32_t *arrived, cudaStream_t stream);
+                            cudaStream_t stream);
 // Load the kernels of every tuner candidate of a variant.
 template <int V>
 void preload_transfer_variant();
@@ -295,13 +296,13 @@ void launch_transfer(int mode, const ParticleSoA &P, int n, const DevClass *clas
                      const float *planes, double *reactions, uint32_t *status, int *cache, cudaStream_t stream,
                      const ForkJoin *fj = nullptr);
 // The opening P2G and `seg` substeps of a small scene or batch in one launch
-// (k_segment), on zeroed pools and an empty table; `arrived` is a zeroed device
-// word.  `sp` carries the one-shot forces of the first substep.  False (nothing
-// launched) where the segment has to run kernel by kernel.
+// (k_segment, which clears table and pools itself).  `sp` carries the one-shot
+// forces of the first substep.  False (nothing launched) where the segment has to
+// run kernel by kernel.
 bool launch_small_segment(const ParticleSoA &P, int n, const DevClass *classes, const GridTable &cur,
                           const GridTable &next, const SimParams &sp, const DevObstacle *obstacles,
                           const float *planes, double *reactions, uint32_t *status, int *cache, int seg,
-                          uint32_t *arrived, cudaStream_t stream);
+                          cudaStream_t stream);
 // Grid update of `g`'s pool; also zeroes the same blocks in `next`'s pool.
 void launch_grid_update(const GridTable &g, const GridTable &next, const SimParams &sp,
                         const DevObstacle *obstacles, const float *planes, double *reactions,

@@ -43,7 +43,10 @@ __global__ void k_clear_table(GridTable g) {
         g.keys[s] = kEmptyKey;
         g.vals[s] = kPendingId;
     }
-    if (gtid == 0) *g.count = 0;
+    if (gtid == 0) {
+        g.count[0] = 0;
+        g.count[kDirtyWord] = ~0u;
+    }
 }
 
 __global__ void k_bin_keys(BinSource src, int32_t *cells, uint32_t *keys, uint32_t *vals) {
@@ -182,13 +185,12 @@ void launch_transfer(int mode, const ParticleSoA &P, int n, const DevClass *clas
 bool launch_small_segment(const ParticleSoA &P, int n, const DevClass *classes, const GridTable &cur,
                           const GridTable &next, const SimParams &sp, const DevObstacle *obstacles,
                           const float *planes, double *reactions, uint32_t *status, int *cache, int seg,
-                          uint32_t *arrived, cudaStream_t stream) {
-    if (n <= 0 || seg <= 0 || !arrived || sp.cpic) return false;
+                          cudaStream_t stream) {
+    if (n <= 0 || seg <= 0 || sp.cpic) return false;
     SimParams one = sp;
     one.defer = nullptr;  // nothing is deferred: every chunk runs the general path
 #define TMPM_VARIANT(V)                                                                                            \
-    launch_segment_variant<V>(P, n, classes, cur, next, one, obstacles, planes, reactions, status, cache, seg, arrived, \
-                              stream)
+    launch_segment_variant<V>(P, n, classes, cur, next, one, obstacles, planes, reactions, status, cache, seg, stream)
     if (sp.multi) return TMPM_VARIANT(kMulti);
     if (sp.has_plastic || sp.num_obstacles > 0) return TMPM_VARIANT(kPlainObst);
     return TMPM_VARIANT(kPlain);

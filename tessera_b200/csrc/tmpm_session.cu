@@ -431,22 +431,22 @@ struct TmpmSession {
         launch_steps(sp, rows, seg, apply_force);
     }
 
-    // The table clear, P2G and substeps of a segment on row buffer `rows`: a
-    // small scene in one launch, otherwise kernel by kernel.
+    // The table clear, P2G and substeps of a segment on row buffer `rows`: one
+    // launch for a small scene, otherwise kernel by kernel.
     void launch_steps(const SimParams &sp, int rows, uint32_t seg, bool apply_force) {
         const int bs = sp.block_shift;
         GridTable g[2];
         grid_views(g, bs);
         const ParticleSoA P = pbuf[rows].view(force.ptr, std::max<size_t>(world.n, 1));
-        launch_clear_table(g[0], g[1], bs, stream);
-        const SimParams sp0 = substep_params(sp, -1, false);
-        open_defer_lists(sp0);
         if (launch_small_segment(P, n_dev, classes.ptr, g[1], g[0], substep_params(sp, -1, apply_force),
                                  dev_obstacles.ptr, dev_planes.ptr, reactions.ptr, status.ptr, cta_cache.ptr,
-                                 static_cast<int>(seg), sp0.defer ? sp0.defer + kBarrierWord : nullptr, stream)) {
+                                 static_cast<int>(seg), stream)) {
             if (apply_force) cudaMemsetAsync(force.ptr, 0, sizeof(float) * force.count, stream);
             return;
         }
+        launch_clear_table(g[0], g[1], bs, stream);
+        const SimParams sp0 = substep_params(sp, -1, false);
+        open_defer_lists(sp0);
         launch_transfer(kModeP2G, P, n_dev, classes.ptr, g[1], g[0], sp0, dev_obstacles.ptr, dev_planes.ptr,
                         reactions.ptr, status.ptr, cta_cache.ptr, stream);
         for (uint32_t k = 0; k < seg; ++k) {
@@ -1089,7 +1089,8 @@ TmpmStatus tmpm_encode_particle_snapshot(TmpmSession *s, void *device_out, size_
     size_t bytes = 32 * s->world.n;
     if (!device_out || capacity_bytes < bytes) return s->fail(TMPM_ERR_CAPACITY, "snapshot buffer too small");
     cudaSetDevice(s->device);
-    cudaMemsetAsync(device_out, 0, bytes, s->stream);
+    // rows of disabled particles read as zero
+    if (static_cast<size_t>(s->n_dev) != s->world.n) cudaMemsetAsync(device_out, 0, bytes, s->stream);
     launch_snapshot(s->soa(), s->n_dev, s->classes.ptr, static_cast<float4 *>(device_out), s->stream);
     cudaError_t e = cudaStreamSynchronize(s->stream);
     if (e) return s->cuda_fail(e, "snapshot");

@@ -40,7 +40,15 @@ constexpr int kTileMaxDim = 64;
 // 1.0 % above 2304; those take the direct path (fused launch 0.428 -> 0.421 ms
 // with the larger tile).
 constexpr int tile_nodes(int threads) { return threads * 9; }
-constexpr int kMaxTileBlocks = kCacheStride - 16;
+// A whole-segment kernel's chunks are alone with one or three others on their SM
+// and share no record with another kernel, so its tile takes what shared memory
+// is left: 22 nodes per particle (88 KB of dynamic shared memory for 256).  A
+// chunk on the direct path (sorted particles that jump between blocks) holds up
+// every barrier of the segment: 16 substeps of the 39,304-particle snow block
+// 593 -> 472 us, of the 55k elastic block 406 -> 403 us, with the larger tile.
+constexpr int segment_tile_nodes(int threads) { return threads * 22; }
+// Blocks a box may span, by its tile's size.
+constexpr int tile_blocks(int threads, int tile) { return tile > tile_nodes(threads) ? kCacheStride - 16 : 128; }
 constexpr int kCacheHeader = 16;
 
 struct Box {
@@ -69,22 +77,32 @@ __device__ __forceinline__ void tile_strides(int d1, int d2, int &s1, int &s2) {
 }
 
 // Split a padded tile index t (strides s1, s2) into (tx, ty, tz) without
-// division: t / d = (t * m) >> 22 with m just above 2^22 / d.  Exact for every
-// tile index: m d - 2^22 < 1.2 d + 1, so the quotient is exact while
-// t (1.2 d + 1) < 2^22, and a box has at least three x planes, so t < 2304 and
-// d <= 768 (t * m < 2^32 with d >= 3).  The approximate reciprocal is off by
-// less than the 0.1 added before truncation.
+// division, with a multiplier just above 2^22 / d (t / d = (t * m) >> 22) or, for
+// a tile of more than 2304 entries, just above 2^32 / d (the high word of t * m).
+// Exact for every tile index.  m d - 2^22 < 1.2 d + 1: the quotient is exact
+// while t (1.2 d + 1) < 2^22, and a box has at least three x planes, so t < 2304
+// and d <= 768 (t * m < 2^32 with d >= 3); the approximate reciprocal is off by
+// less than the 0.1 added before truncation.  m d - 2^32 < 3200 + d: exact while
+// t (3200 + d) < 2^32; the factor 1 + 2^-21 covers the reciprocal's two ulps.
+template <bool WIDE>
 __device__ __forceinline__ unsigned split_factor(int d) {
+    if (WIDE) return static_cast<unsigned>(__fdividef(4294967296.0f, static_cast<float>(d)) * (1.0f + 4.76837158e-7f)) + 1u;
     return static_cast<unsigned>(__fdividef(4194304.0f, static_cast<float>(d)) + 0.1f) + 1u;
 }
+template <bool WIDE>
 struct SplitP {
     int s1, s2;
     unsigned m1, m2;
-    __device__ __forceinline__ SplitP(int s1_, int s2_) : s1(s1_), s2(s2_), m1(split_factor(s1_)), m2(split_factor(s2_)) {}
+    __device__ __forceinline__ SplitP(int s1_, int s2_)
+        : s1(s1_), s2(s2_), m1(split_factor<WIDE>(s1_)), m2(split_factor<WIDE>(s2_)) {}
+    static __device__ __forceinline__ int quotient(int t, unsigned m) {
+        if (WIDE) return static_cast<int>(__umulhi(static_cast<unsigned>(t), m));
+        return static_cast<int>((static_cast<unsigned>(t) * m) >> 22);
+    }
     __device__ __forceinline__ void operator()(int t, int &tx, int &ty, int &tz) const {
-        tx = static_cast<int>((static_cast<unsigned>(t) * m1) >> 22);
+        tx = quotient(t, m1);
         const int r = t - tx * s1;
-        ty = static_cast<int>((static_cast<unsigned>(r) * m2) >> 22);
+        ty = quotient(r, m2);
         tz = r - ty * s2;
     }
 };
@@ -113,7 +131,7 @@ struct Split3 {
 };
 
 // Block-wide min/max of base cells and colours; thread 0 fills `box`.
-template <int THREADS, int BS>
+template <int THREADS, int BS, int TILE>
 __device__ __forceinline__ void reduce_box(bool valid, const int b[3], uint32_t color, int (*red)[8], Box &box) {
     int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int vals[8];
@@ -161,7 +179,7 @@ __device__ __forceinline__ void reduce_box(bool valid, const int b[3], uint32_t 
             box.s1 = s1;
             box.s2 = s2;
             nodes = box.dim[0] * s1;
-            ok = nodes <= tile_nodes(THREADS) && nbt <= kMaxTileBlocks;
+            ok = nodes <= TILE && nbt <= tile_blocks(THREADS, TILE);
         }
         box.nodes = nodes;
         box.nbt = nbt;
@@ -172,7 +190,7 @@ __device__ __forceinline__ void reduce_box(bool valid, const int b[3], uint32_t 
 }
 
 // The box of base cells m[0..2] .. m[3..5] (m[0] > m[3]: no particle), 2 cells wider.
-template <int THREADS, int BS>
+template <int THREADS, int BS, int TILE>
 __device__ __forceinline__ void box_of(const int m[], bool one_color, uint32_t color, Box &box) {
     bool ok = m[0] <= m[3] && one_color;
     int nodes = m[0] <= m[3] ? 1 : 0, nbt = 1;  // nodes 0: no valid particle
@@ -189,7 +207,7 @@ __device__ __forceinline__ void box_of(const int m[], bool one_color, uint32_t c
         }
         tile_strides(box.dim[1], box.dim[2], box.s1, box.s2);
         nodes = box.dim[0] * box.s1;
-        ok = nodes <= tile_nodes(THREADS) && nbt <= kMaxTileBlocks;
+        ok = nodes <= TILE && nbt <= tile_blocks(THREADS, TILE);
     }
     box.nodes = nodes;
     box.nbt = nbt;
@@ -202,7 +220,7 @@ __device__ __forceinline__ void box_of(const int m[], bool one_color, uint32_t c
 // publishes a partial, then every warp combines the partials itself (no second
 // barrier, no shared result).  The maxima are taken on the float bits, whose
 // integer order is the value order for non-negative floats.
-template <int THREADS, int BS>
+template <int THREADS, int BS, int TILE>
 __device__ __forceinline__ void reduce_box_sums(bool valid, const int b[3], uint32_t color, float &sum_a, float &sum_b,
                                                 float &max_a, float &max_b, int (*red)[8], float (*redf)[4],
                                                 Box &box) {
@@ -250,7 +268,7 @@ __device__ __forceinline__ void reduce_box_sums(bool valid, const int b[3], uint
     }
     sum_a = fa;
     sum_b = fb;
-    box_of<THREADS, BS>(m, m[6] == m[7], static_cast<uint32_t>(m[6]), box);
+    box_of<THREADS, BS, TILE>(m, m[6] == m[7], static_cast<uint32_t>(m[6]), box);
 }
 
 // The same for a chunk whose gather used its record: the namespace is the
@@ -262,7 +280,7 @@ __device__ __forceinline__ void reduce_box_sums(bool valid, const int b[3], uint
 __device__ __forceinline__ void chunk_extremes_init(int *ext) {
     if (threadIdx.x < 8) ext[threadIdx.x] = threadIdx.x < 3 ? INT_MAX : (threadIdx.x < 6 ? INT_MIN : 0);
 }
-template <int THREADS, int BS>
+template <int THREADS, int BS, int TILE>
 __device__ __forceinline__ void reduce_box_recorded(bool valid, const int b[3], const Box &gbox, float &sum_p,
                                                     float &max_p, int *ext, float *psum, Box &box) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -291,7 +309,7 @@ __device__ __forceinline__ void reduce_box_recorded(bool valid, const int b[3], 
 #pragma unroll
     for (int w = 1; w < THREADS / 32; ++w) f += psum[w];
     sum_p = f;
-    box_of<THREADS, BS>(m, true, gbox.color, box);
+    box_of<THREADS, BS, TILE>(m, true, gbox.color, box);
 }
 
 // A CTA in which one particle's mass or momentum bound exceeds this share of
@@ -450,27 +468,33 @@ struct TransferSmem {
     Box *box;
     Box *gbox;  // the G2P box, whose block ids the P2G reuses (shared: not held in registers)
     int *abort;
+    int *record;   // a resident chunk's record (else in the cache array)
     int *ext;      // reduce_box_recorded
     float *psum;
     float (*park)[THREADS];  // the affine matrix across the obstacle contact
 };
 // The arrays, one set per kernel for each (THREADS, OBST): the deferred
 // kernel's P2G-only and whole-chunk passes share them.
-template <int THREADS, bool OBST>
+extern __shared__ float4 dynamic_tile[];  // of kernels whose tile exceeds tile_nodes (static shared memory ends at 48 KB)
+template <int THREADS, bool OBST, int TILE>
 __device__ __forceinline__ TransferSmem<THREADS, OBST> transfer_smem() {
-    __shared__ float4 tile[tile_nodes(THREADS)];
+    constexpr bool kDynamic = TILE > tile_nodes(THREADS);
+    constexpr int kBlocks = tile_blocks(THREADS, TILE);
+    __shared__ float4 static_tile[kDynamic ? 1 : TILE];
+    float4 *const tile = kDynamic ? dynamic_tile : static_tile;
     __shared__ float fred[THREADS / 32][4];
-    __shared__ int blk[kMaxTileBlocks];
-    __shared__ int blk2[kMaxTileBlocks];
-    __shared__ int used[kMaxTileBlocks];
+    __shared__ int blk[kBlocks];
+    __shared__ int blk2[kBlocks];
+    __shared__ int used[kBlocks];
     __shared__ int red[THREADS / 32][8];
     __shared__ Box box;
     __shared__ Box gbox;
     __shared__ int abort_flag;
+    __shared__ int record[kDynamic ? kCacheStride : 1];
     __shared__ __align__(16) int ext[8];
     __shared__ __align__(16) float psum[THREADS / 32];
     __shared__ float park[OBST ? 9 : 1][THREADS];
-    return TransferSmem<THREADS, OBST>{tile, fred, blk, blk2, used, red, &box, &gbox, &abort_flag, ext, psum, park};
+    return TransferSmem<THREADS, OBST>{tile, fred, blk, blk2, used, red, &box, &gbox, &abort_flag, record, ext, psum, park};
 }
 
 // Deferred-chunk lists (layout at DeferLists): 0 = P2G only, 1 = whole
@@ -507,9 +531,22 @@ __device__ __forceinline__ int record_tag(int step_index) { return 1 + (step_ind
 // scatters) the fast kernel keeps the common path's values in registers: at
 // 64 registers 24 / 28 bytes of spill stores / loads against 52 / 84 with the
 // fallbacks compiled in.
-template <int MODE, bool PLASTIC, int VARIANT, int THREADS, int BS, bool FAST>
+//
+// RESIDENT (whole-segment kernels: the CTA runs this chunk in every phase): the
+// particle's position, F, plastic state and class word stay in `cs` and the
+// chunk's record in shared memory from the opening P2G (which loads them) to
+// the closing G2P (which stores them).
+struct ChunkState {
+    V3f x;
+    M3f F;
+    float pl[3];
+    uint32_t cw, color;
+    int kind;
+};
+template <int MODE, bool PLASTIC, int VARIANT, int THREADS, int BS, bool FAST, int TILE = tile_nodes(THREADS),
+          bool RESIDENT = false>
 __device__ __forceinline__ void transfer_chunk(TMPM_TRANSFER_PARAMS, const int chunk, const int step_index,
-                                               const int apply_force) {
+                                               const int apply_force, ChunkState *cs = nullptr) {
     constexpr bool MULTI = VARIANT == kMulti;
     constexpr bool CPIC = VARIANT == kCpic;
     constexpr bool OBST = has_obstacles(VARIANT);
@@ -518,8 +555,9 @@ __device__ __forceinline__ void transfer_chunk(TMPM_TRANSFER_PARAMS, const int c
     // and defers a chunk that may touch one.
     constexpr bool CONTACT = OBST && !FAST;
     static_assert(!FAST || (MODE == kModeG2P2G && !CPIC), "the fast path is the fused transfer without CPIC");
-    constexpr int kTileNodes = tile_nodes(THREADS);
-    const TransferSmem<THREADS, CONTACT> S = transfer_smem<THREADS, CONTACT>();
+    constexpr int kTileNodes = TILE;
+    constexpr bool kWideSplit = TILE > 2304;
+    const TransferSmem<THREADS, CONTACT> S = transfer_smem<THREADS, CONTACT, TILE>();
     float4 *const s_gv = S.tile;
     int (*const s_sc)[kTileNodes] = reinterpret_cast<int (*)[kTileNodes]>(S.tile);
     float (*const s_fred)[4] = S.fred;
@@ -536,13 +574,13 @@ __device__ __forceinline__ void transfer_chunk(TMPM_TRANSFER_PARAMS, const int c
     const int i = chunk * THREADS + static_cast<int>(threadIdx.x);
     const uint32_t off = static_cast<uint32_t>(i) * 4u;
     const bool valid = i < n;
-    int *const cc = cache + static_cast<size_t>(chunk) * kCacheStride;
+    int *const cc = RESIDENT ? S.record : cache + static_cast<size_t>(chunk) * kCacheStride;
 
     if (threadIdx.x == 0) s_abort = (*reinterpret_cast<volatile uint32_t *>(status) & kFatal) != 0;
     if (MODE != kModeG2P) {
         // The first barrier of the kernel orders these.
         if (MODE == kModeG2P2G) chunk_extremes_init(S.ext);
-        for (int t = threadIdx.x; t < kMaxTileBlocks; t += THREADS) s_used[t] = 0;
+        for (int t = threadIdx.x; t < tile_blocks(THREADS, TILE); t += THREADS) s_used[t] = 0;
     }
 
     V3f x = mk(0, 0, 0);
@@ -551,7 +589,12 @@ __device__ __forceinline__ void transfer_chunk(TMPM_TRANSFER_PARAMS, const int c
     DevClass k;
     k.mass = 0.f;
     k.color = 0;
-    if (valid) {
+    if (RESIDENT && MODE != kModeP2G) {
+        x = cs->x;
+        cw = cs->cw;
+        k.color = cs->color;
+        k.kind = cs->kind;
+    } else if (valid) {
         x = load_v3(P.x, cap, off);
         cw = P.cls[i];
         // the namespace and kind now; the whole record after the gather (below)
@@ -581,7 +624,10 @@ __device__ __forceinline__ void transfer_chunk(TMPM_TRANSFER_PARAMS, const int c
     const bool isotropic = fluid && (MODE == kModeP2G ? step_index >= 0 : step_index > 0);
     const bool plastic = PLASTIC && g2p_on && k.kind >= kMatSnow;
     float pl[3] = {1.0f, 0.0f, 0.0f};
-    if (plastic) {
+    if (RESIDENT && MODE != kModeP2G) {
+        if (PLASTIC)
+            for (int q = 0; q < 3; ++q) pl[q] = cs->pl[q];
+    } else if (plastic) {
         const V3f q = load_v3(P.pl, cap, off);
         pl[0] = q.x;
         pl[1] = q.y;
@@ -597,6 +643,7 @@ __device__ __forceinline__ void transfer_chunk(TMPM_TRANSFER_PARAMS, const int c
             load_deformation(P.F, cap, off, isotropic, F);
             k = classes[cw & kClassMask];
         }
+        if (RESIDENT) *cs = ChunkState{x, F, {pl[0], pl[1], pl[2]}, cw, k.color, k.kind};
         if (p2g_on) {
             v = load_v3(P.v, cap, off);
             Cm = load_m3(P.C, cap, off);
@@ -639,7 +686,7 @@ __device__ __forceinline__ void transfer_chunk(TMPM_TRANSFER_PARAMS, const int c
                 bx.ok = 0;
                 bx.color = 0;
             } else if constexpr (!FAST) {
-                reduce_box<THREADS, BS>(g2p_on, b, ns, s_red, s_box);
+                reduce_box<THREADS, BS, TILE>(g2p_on, b, ns, s_red, s_box);
                 bx = s_box;
                 if (bx.ok) {
                     const Split3 split(bx.nb[1], bx.nb[2]);
@@ -655,22 +702,35 @@ __device__ __forceinline__ void transfer_chunk(TMPM_TRANSFER_PARAMS, const int c
                        (b[0] < bx.lo[0] || b[1] < bx.lo[1] || b[2] < bx.lo[2] || b[0] + 2 >= bx.lo[0] + bx.dim[0] ||
                         b[1] + 2 >= bx.lo[1] + bx.dim[1] || b[2] + 2 >= bx.lo[2] + bx.dim[2] || ns != bx.color);
             if (bx.ok && !bad) {
-                const SplitP split(bx.s1, bx.s2);
-                for (int t = threadIdx.x; t < bx.nodes; t += THREADS) {
+                // four z-consecutive entries per step (the y stride is a multiple
+                // of four): one index split for the four
+                const SplitP<kWideSplit> split(bx.s1, bx.s2);
+                for (int t = 4 * threadIdx.x; t < bx.nodes; t += 4 * THREADS) {
                     int tx, ty, tz;
                     split(t, tx, ty, tz);
-                    if (ty >= bx.dim[1] || tz >= bx.dim[2]) continue;  // padding
-                    int cx = bx.lo[0] + tx, cy = bx.lo[1] + ty, cz = bx.lo[2] + tz;
-                    int tb = tile_block_index<BS>(bx, cx, cy, cz);
-                    int id = use_cache ? cc[kCacheHeader + tb] : s_blk[tb];
-                    if (use_cache) s_blk[tb] = id;
-                    if (id >= 0) {
-                        // asynchronous 16-byte copy global -> shared (L2 only), no register staging
-                        const float4 *src = cur.pool + static_cast<size_t>(id) * (1 << (3 * BS)) + node_local<BS>(cx, cy, cz);
-                        const unsigned dst = static_cast<unsigned>(__cvta_generic_to_shared(s_gv + t));
-                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
-                    } else {
-                        s_gv[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (ty >= bx.dim[1]) continue;  // padding
+                    const int cx = bx.lo[0] + tx, cy = bx.lo[1] + ty;
+                    const int tb0 = tile_block_index<BS>(bx, cx, cy, bx.blo[2] << BS);
+                    const int local = node_local<BS>(cx, cy, 0);
+                    const unsigned dst = static_cast<unsigned>(__cvta_generic_to_shared(s_gv + t));
+                    int id = -1;
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        if (tz + e >= bx.dim[2]) break;  // padding
+                        const int cz = bx.lo[2] + tz + e;
+                        if (e == 0 || (cz & ((1 << BS) - 1)) == 0) {
+                            const int tb = tb0 + (cz >> BS) - bx.blo[2];
+                            id = use_cache ? cc[kCacheHeader + tb] : s_blk[tb];
+                            if (use_cache) s_blk[tb] = id;
+                        }
+                        if (id >= 0) {
+                            // asynchronous 16-byte copy global -> shared (L2 only), no register staging
+                            const float4 *src = cur.pool + (static_cast<size_t>(id) << (3 * BS)) +
+                                                (local + (cz & ((1 << BS) - 1)));
+                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * e), "l"(src) : "memory");
+                        } else {
+                            s_gv[t + e] = make_float4(0.f, 0.f, 0.f, 0.f);
+                        }
                     }
                 }
                 asm volatile("cp.async.wait_all;" ::: "memory");
@@ -774,7 +834,8 @@ __device__ __forceinline__ void transfer_chunk(TMPM_TRANSFER_PARAMS, const int c
         // live is saved) an updating particle reads F after the contact.
         const bool updates = g2p_on && !fixed;
         if (valid) {
-            if (!CONTACT || !updates) load_deformation(P.F, cap, off, isotropic, F);
+            if (RESIDENT) F = cs->F;
+            else if (!CONTACT || !updates) load_deformation(P.F, cap, off, isotropic, F);
             k = classes[cw & kClassMask];
         }
         V3f pos = x;
@@ -854,7 +915,10 @@ __device__ __forceinline__ void transfer_chunk(TMPM_TRANSFER_PARAMS, const int c
             }
         }
         if (updates) {
-            if (CONTACT) load_deformation(P.F, cap, off, isotropic, F);
+            if (CONTACT) {
+                if (RESIDENT) F = cs->F;
+                else load_deformation(P.F, cap, off, isotropic, F);
+            }
             const M3f grad = add(m3_identity(), scale(aff, dt));  // F <- (I + dt C) F
             M3f Fn;
             bool plastic_ok = true;
@@ -901,9 +965,15 @@ __device__ __forceinline__ void transfer_chunk(TMPM_TRANSFER_PARAMS, const int c
             Cm = aff;
             F = Fn;
         }
-        if (g2p_on) {
+        const bool last = MODE == kModeG2P || (MULTI && !p2g_on);
+        if (RESIDENT && MODE != kModeG2P) {
+            cs->x = x;
+            cs->F = F;
+            if (PLASTIC)
+                for (int q = 0; q < 3; ++q) cs->pl[q] = pl[q];
+        }
+        if (g2p_on && (!RESIDENT || last)) {
             store_v3(P.x, cap, off, x);
-            const bool last = MODE == kModeG2P || (MULTI && !p2g_on);
             if (!fixed) {
                 if (fluid && step_index > 0 && !last) store_row(P.F, cap, 0, off, F.c0.x);
                 else store_m3(P.F, cap, off, F);
@@ -958,10 +1028,10 @@ __device__ __forceinline__ void transfer_chunk(TMPM_TRANSFER_PARAMS, const int c
         // the record's P2G summed the masses of these particles (or of a
         // superset that bounds them) and found none dominant
         sm = __int_as_float(cc[15]);
-        reduce_box_recorded<THREADS, BS>(active, b, s_gbox, tot_p, max_p, S.ext, S.psum, bx);
+        reduce_box_recorded<THREADS, BS, TILE>(active, b, s_gbox, tot_p, max_p, S.ext, S.psum, bx);
     } else {
         float tot_m = bound_m, max_m = bound_m;
-        reduce_box_sums<THREADS, BS>(active, b, ns, tot_m, tot_p, max_m, max_p, s_red, s_fred, bx);
+        reduce_box_sums<THREADS, BS, TILE>(active, b, ns, tot_m, tot_p, max_m, max_p, s_red, s_fred, bx);
         sm = pow2_scale(tot_m);
         if (max_m > tot_m * kFloatModeShare) bx.ok = 0;
     }
@@ -1091,19 +1161,31 @@ __device__ __forceinline__ void transfer_chunk(TMPM_TRANSFER_PARAMS, const int c
         }
         __syncthreads();
         const float inv_sm = pow2_inverse(sm), inv_sp = pow2_inverse(spv);
-        const SplitP split_n(bx.s1, bx.s2);
-        for (int t = threadIdx.x; t < bx.nodes; t += THREADS) {
-            const int m = s_sc[0][t], px = s_sc[1][t], py = s_sc[2][t], pz = s_sc[3][t];
-            if ((m | px | py | pz) == 0) continue;  // also every padding entry
+        const SplitP<kWideSplit> split_n(bx.s1, bx.s2);
+        for (int t = 4 * threadIdx.x; t < bx.nodes; t += 4 * THREADS) {  // four entries per step, as the fill
+            const int4 m = *reinterpret_cast<const int4 *>(&s_sc[0][t]), px = *reinterpret_cast<const int4 *>(&s_sc[1][t]),
+                       py = *reinterpret_cast<const int4 *>(&s_sc[2][t]), pz = *reinterpret_cast<const int4 *>(&s_sc[3][t]);
+            const int any[4] = {m.x | px.x | py.x | pz.x, m.y | px.y | py.y | pz.y, m.z | px.z | py.z | pz.z,
+                                m.w | px.w | py.w | pz.w};
+            if ((any[0] | any[1] | any[2] | any[3]) == 0) continue;
             int tx, ty, tz;
             split_n(t, tx, ty, tz);
-            if (ty >= bx.dim[1] || tz >= bx.dim[2]) continue;  // padding (zero by construction; never flushed)
-            int cx = bx.lo[0] + tx, cy = bx.lo[1] + ty, cz = bx.lo[2] + tz;
-            int id = s_blk2[tile_block_index<BS>(bx, cx, cy, cz)];
-            if (id < 0) continue;
-            atomicAdd(next.pool + static_cast<size_t>(id) * (1 << (3 * BS)) + node_local<BS>(cx, cy, cz),
-                      make_float4(static_cast<float>(m) * inv_sm, static_cast<float>(px) * inv_sp,
-                                  static_cast<float>(py) * inv_sp, static_cast<float>(pz) * inv_sp));
+            if (ty >= bx.dim[1]) continue;  // padding (zero by construction; never flushed)
+            const int cx = bx.lo[0] + tx, cy = bx.lo[1] + ty;
+            const int tb0 = tile_block_index<BS>(bx, cx, cy, bx.blo[2] << BS);
+            const int local = node_local<BS>(cx, cy, 0);
+            const int ms[4] = {m.x, m.y, m.z, m.w}, xs[4] = {px.x, px.y, px.z, px.w}, ys[4] = {py.x, py.y, py.z, py.w},
+                      zs[4] = {pz.x, pz.y, pz.z, pz.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                if (any[e] == 0 || tz + e >= bx.dim[2]) continue;
+                const int cz = bx.lo[2] + tz + e;
+                const int id = s_blk2[tb0 + (cz >> BS) - bx.blo[2]];
+                if (id < 0) continue;
+                atomicAdd(next.pool + (static_cast<size_t>(id) << (3 * BS)) + (local + (cz & ((1 << BS) - 1))),
+                          make_float4(static_cast<float>(ms[e]) * inv_sm, static_cast<float>(xs[e]) * inv_sp,
+                                      static_cast<float>(ys[e]) * inv_sp, static_cast<float>(zs[e]) * inv_sp));
+            }
         }
     } else {
         if (threadIdx.x == 0) {
@@ -1182,49 +1264,68 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? TMPM_TRANSFER_MIN_BL
     }
 }
 
-// A whole segment of a small scene (or batch) in one cooperative launch: the
-// opening P2G, then `seg` substeps of grid update and fused transfer, the last
-// one G2P-only, with a grid-wide barrier between phases.
+// A whole segment of a small scene (or batch) in one cooperative launch: table
+// and pools cleared, the opening P2G, then `seg` substeps of grid update and
+// fused transfer, the last one G2P-only, with a grid-wide barrier between
+// phases; CTA c runs chunk c in every phase.
 //
 // At these sizes a substep's kernels are each a partial wave and the time goes
-// into launches, the fork and join of the deferred chunks and the tails of
-// dependent kernels; every phase here starts one barrier after the last.  All
-// chunks take the general path (there are registers for it at two CTAs of 256
-// particles an SM), so nothing is deferred.  Chunk c belongs to CTA c %
-// gridDim.x in every phase: particle rows and the chunk's record are only read
-// by the SM that wrote them; grid data is read through L2.
+// into launches, the fork and join of the deferred chunks, the tails of
+// dependent kernels and round trips to L2 for state the SM just wrote.  Here a
+// phase starts one barrier after the last, the particle's state stays in
+// registers and the chunk's record in shared memory, and only the grid goes
+// through L2.  All chunks take the general path (128 registers a thread at two
+// CTAs of 256 particles an SM), so nothing is deferred.  A frame of
+// 8 substeps of 512 particles: 171 -> 139 us with the state and record kept and
+// the clears inside (a substep 29,300 -> 22,900 cycles); of 16 substeps of 54,872
+// particles 403 -> 341 us, 39,304 of snow 472 -> 399 us (kernel by kernel: 176,
+// 483 and 613 us).
 template <bool PLASTIC, int VARIANT, int THREADS, int BS>
-__global__ void __launch_bounds__(THREADS, kSegmentThreads / THREADS)
-    k_segment(TMPM_TRANSFER_PARAMS, int seg, uint32_t *arrived) {
-    const int chunks = (n + THREADS - 1) / THREADS;
-    uint32_t target = 0;
-    for (int c = blockIdx.x; c < chunks; c += gridDim.x) {
-        __syncthreads();
-        transfer_chunk<kModeP2G, PLASTIC, VARIANT, THREADS, BS, false>(TMPM_TRANSFER_ARGS, c, -1, 0);
+__global__ void __launch_bounds__(THREADS, kSegmentThreads / THREADS) k_segment(TMPM_TRANSFER_PARAMS, int seg) {
+    constexpr int TILE = segment_tile_nodes(THREADS);
+    uint32_t *const arrived = cur.count + kBarrierWord;
+    const size_t gtid = static_cast<size_t>(blockIdx.x) * THREADS + threadIdx.x;
+    const size_t stride = static_cast<size_t>(gridDim.x) * THREADS;
+    const int chunk = blockIdx.x;
+    {
+        const size_t dirty = min(static_cast<size_t>(__ldcg(cur.count + kDirtyWord)), cur.pool_nodes);
+        for (size_t t = gtid; t < dirty; t += stride) {
+            cur.pool[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+            next.pool[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        for (size_t t = gtid; t <= cur.mask; t += stride) {
+            cur.keys[t] = kEmptyKey;
+            cur.vals[t] = kPendingId;
+        }
+        if (gtid == 0) *cur.count = 0;
     }
+    uint32_t target = gridDim.x;
+    if (!grid_barrier(arrived, target, status)) return;
+    ChunkState cs;
+    transfer_chunk<kModeP2G, PLASTIC, VARIANT, THREADS, BS, false, TILE, true>(TMPM_TRANSFER_ARGS, chunk, -1, 0, &cs);
     GridTable a = next, b = cur;  // one table, two pools: `a` holds the nodes of the substep at hand
     for (int k = 0; k < seg; ++k) {
-        target += gridDim.x;
-        if (!grid_barrier(arrived, target, status)) return;
+        if (!grid_barrier(arrived, target += gridDim.x, status)) return;
         if (!(*reinterpret_cast<volatile uint32_t *>(status) & kFatal))
-            grid_nodes<VARIANT == kMulti, BS, has_obstacles(VARIANT)>(
-                a, b.pool, sp, obstacles, planes, reactions, static_cast<size_t>(blockIdx.x) * THREADS + threadIdx.x,
-                static_cast<size_t>(gridDim.x) * THREADS);
-        target += gridDim.x;
-        if (!grid_barrier(arrived, target, status)) return;
+            grid_nodes<VARIANT == kMulti, BS, has_obstacles(VARIANT)>(a, b.pool, sp, obstacles, planes, reactions, gtid,
+                                                                      stride);
+        if (!grid_barrier(arrived, target += gridDim.x, status)) return;
         const int force = k == 0 ? sp.apply_force : 0;
-        for (int c = blockIdx.x; c < chunks; c += gridDim.x) {
-            __syncthreads();
-            if (k + 1 < seg)
-                transfer_chunk<kModeG2P2G, PLASTIC, VARIANT, THREADS, BS, false>(
-                    P, n, classes, a, b, sp, obstacles, planes, reactions, status, cache, c, k, force);
-            else
-                transfer_chunk<kModeG2P, PLASTIC, VARIANT, THREADS, BS, false>(
-                    P, n, classes, a, b, sp, obstacles, planes, reactions, status, cache, c, k, force);
-        }
+        if (k + 1 < seg)
+            transfer_chunk<kModeG2P2G, PLASTIC, VARIANT, THREADS, BS, false, TILE, true>(
+                P, n, classes, a, b, sp, obstacles, planes, reactions, status, cache, chunk, k, force, &cs);
+        else
+            transfer_chunk<kModeG2P, PLASTIC, VARIANT, THREADS, BS, false, TILE, true>(
+                P, n, classes, a, b, sp, obstacles, planes, reactions, status, cache, chunk, k, force, &cs);
         float4 *const pool = a.pool;
         a.pool = b.pool;
         b.pool = pool;
+    }
+    if (gtid == 0) cur.count[kDirtyWord] = min(__ldcg(cur.count), cur.max_blocks) << (3 * BS);
+    // the last CTA past every barrier leaves their words at zero
+    if (threadIdx.x == 0 && atomicAdd(cur.count + kExitWord, 1u) == gridDim.x - 1) {
+        *arrived = 0;
+        cur.count[kExitWord] = 0;
     }
 }
 #undef TMPM_TRANSFER_ARGS
@@ -1316,19 +1417,21 @@ namespace {
 template <bool PL, int V, int T, int BS>
 bool try_segment(const ParticleSoA &P, int n, const DevClass *classes, const GridTable &cur, const GridTable &next,
                  const SimParams &sp, const DevObstacle *obstacles, const float *planes, double *reactions,
-                 uint32_t *status, int *cache, int seg, uint32_t *arrived, cudaStream_t stream) {
+                 uint32_t *status, int *cache, int seg, cudaStream_t stream) {
     const int chunks = (n + T - 1) / T;
+    const int smem = segment_tile_nodes(T) * static_cast<int>(sizeof(float4));
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_segment<PL, V, T, BS>, T, 0) != cudaSuccess) {
+    if (cudaFuncSetAttribute(k_segment<PL, V, T, BS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_segment<PL, V, T, BS>, T, smem) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
     const int room = per_sm * device_sm_count();
-    if (room <= 0 || chunks > kSegmentChunksPerCta * room) return false;
+    if (chunks > room) return false;
     void *args[] = {const_cast<ParticleSoA *>(&P), &n, &classes, const_cast<GridTable *>(&cur),
                     const_cast<GridTable *>(&next), const_cast<SimParams *>(&sp), &obstacles, &planes, &reactions,
-                    &status, &cache, &seg, &arrived};
-    if (cudaLaunchCooperativeKernel(k_segment<PL, V, T, BS>, dim3(std::min(chunks, room)), dim3(T), args, 0, stream) ==
+                    &status, &cache, &seg};
+    if (cudaLaunchCooperativeKernel(k_segment<PL, V, T, BS>, dim3(chunks), dim3(T), args, smem, stream) ==
         cudaSuccess)
         return true;
     cudaGetLastError();
@@ -1340,9 +1443,9 @@ template <int V>
 bool launch_segment_variant(const ParticleSoA &P, int n, const DevClass *classes, const GridTable &cur,
                             const GridTable &next, const SimParams &sp, const DevObstacle *obstacles,
                             const float *planes, double *reactions, uint32_t *status, int *cache, int seg,
-                            uint32_t *arrived, cudaStream_t stream) {
+                            cudaStream_t stream) {
 #define TMPM_SEGMENT(PL, T, BS) \
-    try_segment<PL, V, T, BS>(P, n, classes, cur, next, sp, obstacles, planes, reactions, status, cache, seg, arrived, stream)
+    try_segment<PL, V, T, BS>(P, n, classes, cur, next, sp, obstacles, planes, reactions, status, cache, seg, stream)
     if (sp.has_plastic) {
         if constexpr (V == kPlainObst) return TMPM_SEGMENT(true, 256, kBlockShift);
         return false;
@@ -1388,6 +1491,6 @@ void preload_transfer_variant() {
 #define TMPM_SEGMENT_VARIANT(V)                                                                                      \
     template bool launch_segment_variant<V>(const ParticleSoA &, int, const DevClass *, const GridTable &,           \
                                             const GridTable &, const SimParams &, const DevObstacle *, const float *, \
-                                            double *, uint32_t *, int *, int, uint32_t *, cudaStream_t);
+                                            double *, uint32_t *, int *, int, cudaStream_t);
 
 }  // namespace tmpm

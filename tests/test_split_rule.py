@@ -7,7 +7,7 @@ import struct
 import numpy as np
 import pytest
 
-TILE = 2304  # entries of the largest tile
+TILE, WIDE_TILE = 2304, 5632  # entries of the largest static tile, of a whole-segment kernel's
 FACTOR_ULPS = 2  # documented error bound of the approximate division
 
 
@@ -29,6 +29,20 @@ def test_split_is_exact_for_every_tile_stride(first, step, last):
         for m in split_factors(d):
             assert (t * np.uint64(m)).max() < 2**32
             assert np.array_equal((t * np.uint64(m)) >> np.uint64(22), t // np.uint64(d)), (d, m)
+
+
+@pytest.mark.parametrize("first,step,last", [(4, 8, 68), (16, 32, WIDE_TILE // 3)])
+def test_wide_split_is_exact_for_every_tile_stride(first, step, last):
+    t = np.arange(WIDE_TILE, dtype=np.uint64)
+    for d in range(first, last + 1, step):
+        lo = hi = np.float32(4294967296.0 / d)
+        for _ in range(FACTOR_ULPS):
+            lo, hi = np.nextafter(lo, np.float32(0)), np.nextafter(hi, np.float32(np.inf))
+        q = lo
+        while q <= hi:
+            m = int(np.float32(q * np.float32(1.0 + 4.76837158e-7))) + 1
+            assert m < 2**32 and np.array_equal((t * np.uint64(m)) >> np.uint64(32), t // np.uint64(d)), (d, m)
+            q = np.nextafter(q, np.float32(np.inf))
 
 
 def bits(x):
