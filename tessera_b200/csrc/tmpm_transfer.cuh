@@ -510,6 +510,11 @@ __device__ __forceinline__ void defer_push(const SimParams &sp, int list, int ch
 // their records meanwhile: the tag keeps the fast kernel from reading them
 // as records of its own step.
 __device__ __forceinline__ int record_tag(int step_index) { return 1 + (step_index & 1); }
+// Added to the tag of a chunk whose particles are near an obstacle: the fast
+// kernel would defer it whole, to run after it; with this bit the chunk is on the
+// no-record list, and the general path runs it beside the fast kernel (with its
+// record).  529k-particle dam break against a sphere, 32 substeps: 2.86 -> 2.28 ms.
+constexpr int kRecordNear = 4;
 
 #define TMPM_TRANSFER_PARAMS \
     ParticleSoA P, int n, const DevClass *__restrict__ classes, GridTable cur, GridTable next, SimParams sp, \
@@ -658,7 +663,8 @@ __device__ __forceinline__ void transfer_chunk(TMPM_TRANSFER_PARAMS, const int c
         // The negative tag says that the P2G took the direct path: so does the
         // gather, without another box reduction.
         const int record = cc[0];
-        bool use_cache = record == record_tag(step_index);
+        bool use_cache = record == record_tag(step_index) ||
+                         (CONTACT && record == (record_tag(step_index) | kRecordNear));
         if constexpr (FAST) {
             if (!use_cache) return;  // on the no-record list (CTA-uniform)
         }
@@ -1056,6 +1062,18 @@ __device__ __forceinline__ void transfer_chunk(TMPM_TRANSFER_PARAMS, const int c
             return;
         }
     }
+    // A chunk that may touch an obstacle in the next substep, a quarter cell away
+    // at most (CTA-uniform).
+    bool near = false;
+    if constexpr (CONTACT && !CPIC) {
+        if (bx.ok && sp.defer && sp.num_obstacles > 0) {
+            if (active) {
+                const float r = k.radius * 1.0001f + 0.25f * h;
+                for (int oi = 0; oi < sp.num_obstacles; ++oi) near = near || obstacle_near(obstacles[oi], x, r);
+            }
+            near = __syncthreads_or(near) != 0;
+        }
+    }
     if (bx.ok) {
         // every warp has finished its gather (barrier above): the buffer becomes the scatter tile
         // (a multiple of 16 entries: the x stride is)
@@ -1142,7 +1160,8 @@ __device__ __forceinline__ void transfer_chunk(TMPM_TRANSFER_PARAMS, const int c
             cc[kCacheHeader + t] = id;
         }
         if (threadIdx.x == 0) {
-            cc[0] = record_tag(step_index + 1);
+            cc[0] = record_tag(step_index + 1) | (near ? kRecordNear : 0);
+            if (near) defer_push(sp, 2 + ((step_index + 1) & 1), chunk);
             cc[1] = bx.blo[0];
             cc[2] = bx.blo[1];
             cc[3] = bx.blo[2];
