@@ -231,6 +231,18 @@ struct ParticleSoA {
     size_t force_stride;
 };
 
+// Lane l of a transfer warp takes the particles of the chunk's cell group
+// lane_cell(l).  With 8 particles per cell the 32 groups of a chunk are 32
+// cells in Morton order, a 2 x 4 x 4 block (x, y, z); the permutation hands
+// each quarter-warp (the 8 lanes of one 128-bit shared-memory phase) a 1 x 2 x 4
+// slab of it.  With the tile strides of tile_strides (y stride 4 mod 8, x
+// stride 16 mod 32) the quarter-warp's gather loads then fall into distinct
+// bank groups, and the warp's 32 scatter atomics into distinct banks.
+__host__ __device__ inline int lane_cell(int l) {
+    const int p = l >> 3, q = l & 7;
+    return (p & 1) * 16 + ((q >> 1) & 1) * 8 + (p >> 1) * 4 + (q >> 2) * 2 + (q & 1);
+}
+
 struct SortBuffers {
     uint32_t *keys[2];
     uint32_t *vals[2];

@@ -64,18 +64,6 @@ __global__ void k_bin_keys(BinSource src, int32_t *cells, uint32_t *keys, uint32
 // (cell-sorted: one or two cells each) and their stencils do not collide on
 // the same shared-memory node.  The last, partial chunk is stored in sorted
 // order.
-// Lane l of a transfer warp takes the particles of the chunk's cell group
-// lane_cell(l).  With 8 particles per cell the 32 groups of a chunk are 32
-// cells in Morton order, a 2 x 4 x 4 block (x, y, z); the permutation hands
-// each quarter-warp (the 8 lanes of one 128-bit shared-memory phase) a 1 x 2 x 4
-// slab of it.  With the tile strides of tile_strides (y stride 4 mod 8, x
-// stride 16 mod 32) the quarter-warp's gather loads then fall into distinct
-// bank groups, and the warp's 32 scatter atomics into distinct banks.
-__device__ __forceinline__ int lane_cell(int l) {
-    const int p = l >> 3, q = l & 7;
-    return (p & 1) * 16 + ((q >> 1) & 1) * 8 + (p >> 1) * 4 + (q >> 2) * 2 + (q & 1);
-}
-
 __global__ void k_gather(ParticleSoA src, ParticleSoA dst, const uint32_t *__restrict__ perm, int n, int interleave) {
     int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
@@ -192,7 +180,9 @@ bool launch_small_segment(const ParticleSoA &P, int n, const DevClass *classes, 
 #define TMPM_VARIANT(V)                                                                                            \
     launch_segment_variant<V>(P, n, classes, cur, next, one, obstacles, planes, reactions, status, cache, seg, stream)
     if (sp.multi) return TMPM_VARIANT(kMulti);
-    if (sp.has_plastic || sp.num_obstacles > 0) return TMPM_VARIANT(kPlainObst);
+    // plastic state without obstacles: the contact's out-of-line call takes
+    // registers the return map needs (864 -> 336 bytes of stack)
+    if (sp.num_obstacles > 0) return TMPM_VARIANT(kPlainObst);
     return TMPM_VARIANT(kPlain);
 #undef TMPM_VARIANT
 }

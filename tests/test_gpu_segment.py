@@ -84,3 +84,33 @@ def test_fluid_deformation_of_uneven_batch_scenes():
         for _ in range(2 * steps[sid]):
             cpu.substep_fixed(5e-5)
         check(cpu, batch.particles(sid), 2 * steps[sid])
+
+
+def test_sessions_of_several_threads_share_the_gpu():
+    """Whole-segment launches of several sessions, each on its own stream from its
+    own thread, with more particles between them than the GPU holds at once: every
+    session gets the result it gets alone."""
+    import threading
+
+    made = [scenes.elastic_block(seed=k, lo=(0.3, 0.3, 0.3), hi=(0.3 + s, 0.3 + s, 0.3 + s)) for k, s in
+            ((1, 0.3), (2, 0.28), (3, 0.1))]
+
+    def frames(sc, out, k):
+        s = Session(sc.params, sc.particles, sc.dt, launch_shape=0)
+        for _ in range(12):
+            s.submit_steps(16)
+        s.synchronize()
+        out[k] = s.particles()
+
+    alone, together = [None] * 3, [None] * 3
+    for k, sc in enumerate(made):
+        frames(sc, alone, k)
+    threads = [threading.Thread(target=frames, args=(sc, together, k)) for k, sc in enumerate(made)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for a, b in zip(alone, together):
+        # 192 substeps apart only by the order of the f32 node sums
+        assert np.abs(a.position - b.position).max() < 4e-5
+        assert np.abs(a.velocity - b.velocity).max() < 4e-4 * max(1.0, np.abs(a.velocity).max())
