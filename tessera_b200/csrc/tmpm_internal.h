@@ -70,6 +70,11 @@ constexpr int config_block_shift(int c) { return c < kNumLaunchShapes ? kBlockSh
 // at once: 75,776 particles on 148 SMs.  Above, kernel by kernel is faster
 // (85,184 particles: 30.1 us a substep against 34.1 with two chunks a CTA).
 constexpr int kSegmentThreads = 512;
+// It launches at least this many threads: the grid update of a few chunks would
+// otherwise walk its blocks with a few hundred (512 particles 12.1 -> 11.4 us a
+// substep, 11.8 -> 10.5 with CTAs of 128; 37,888 threads give it back to the
+// barriers).
+constexpr int kSegmentMinThreads = 8192;
 constexpr int kBarrierSpins = 1 << 24;  // bounded wait at its barriers (a few seconds)
 constexpr int kMinTransferThreads = 128;  // per-CTA records are sized for the smallest shape
 constexpr int kCacheStride = 272;      // per-CTA record: 16-int box header + up to 256 block ids

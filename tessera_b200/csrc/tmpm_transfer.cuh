@@ -1217,7 +1217,9 @@ __global__ void __launch_bounds__(THREADS, kSegmentThreads / THREADS) k_segment(
     uint32_t *const arrived = cur.count + kBarrierWord;
     const size_t gtid = static_cast<size_t>(blockIdx.x) * THREADS + threadIdx.x;
     const size_t stride = static_cast<size_t>(gridDim.x) * THREADS;
+    // CTAs above the chunk count only clear and update the grid
     const int chunk = blockIdx.x;
+    const bool has_chunk = chunk * THREADS < n;
     {
         const size_t dirty = min(static_cast<size_t>(__ldcg(cur.count + kDirtyWord)), cur.pool_nodes);
         for (size_t t = gtid; t < dirty; t += stride) {
@@ -1233,7 +1235,8 @@ __global__ void __launch_bounds__(THREADS, kSegmentThreads / THREADS) k_segment(
     uint32_t target = gridDim.x;
     if (!grid_barrier(arrived, target, status)) return;
     ChunkState cs;
-    transfer_chunk<kModeP2G, PLASTIC, VARIANT, THREADS, BS, false, TILE, true>(TMPM_TRANSFER_ARGS, chunk, -1, 0, &cs);
+    if (has_chunk)
+        transfer_chunk<kModeP2G, PLASTIC, VARIANT, THREADS, BS, false, TILE, true>(TMPM_TRANSFER_ARGS, chunk, -1, 0, &cs);
     GridTable a = next, b = cur;  // one table, two pools: `a` holds the nodes of the substep at hand
     for (int k = 0; k < seg; ++k) {
         if (!grid_barrier(arrived, target += gridDim.x, status)) return;
@@ -1242,10 +1245,10 @@ __global__ void __launch_bounds__(THREADS, kSegmentThreads / THREADS) k_segment(
                                                                       stride);
         if (!grid_barrier(arrived, target += gridDim.x, status)) return;
         const int force = k == 0 ? sp.apply_force : 0;
-        if (k + 1 < seg)
+        if (has_chunk && k + 1 < seg)
             transfer_chunk<kModeG2P2G, PLASTIC, VARIANT, THREADS, BS, false, TILE, true>(
                 P, n, classes, a, b, sp, obstacles, planes, reactions, status, cache, chunk, k, force, &cs);
-        else
+        else if (has_chunk)
             transfer_chunk<kModeG2P, PLASTIC, VARIANT, THREADS, BS, false, TILE, true>(
                 P, n, classes, a, b, sp, obstacles, planes, reactions, status, cache, chunk, k, force, &cs);
         float4 *const pool = a.pool;
@@ -1362,7 +1365,7 @@ bool try_segment(const ParticleSoA &P, int n, const DevClass *classes, const Gri
     void *args[] = {const_cast<ParticleSoA *>(&P), &n, &classes, const_cast<GridTable *>(&cur),
                     const_cast<GridTable *>(&next), const_cast<SimParams *>(&sp), &obstacles, &planes, &reactions,
                     &status, &cache, &seg};
-    if (cudaLaunchCooperativeKernel(k_segment<PL, V, T, BS>, dim3(chunks), dim3(T), args, smem, stream) ==
+    if (cudaLaunchCooperativeKernel(k_segment<PL, V, T, BS>, dim3(std::min(room, std::max(chunks, kSegmentMinThreads / T))), dim3(T), args, smem, stream) ==
         cudaSuccess)
         return true;
     cudaGetLastError();
