@@ -606,31 +606,31 @@ struct TmpmSession {
                 if (!kernel_ms) {
                     launch_steps(sp, resort ? cur ^ 1 : cur, seg, apply_force);
                 } else {
-                GridTable g[2];
-                grid_views(g, bs);
-                const ParticleSoA P = pbuf[resort ? cur ^ 1 : cur].view(force.ptr, std::max<size_t>(world.n, 1));
-                tick(0);
-                launch_clear_table(g[0], g[1], bs, stream);
-                const SimParams sp0 = substep_params(sp, -1, false);
-                open_defer_lists(sp0);
-                launch_transfer(kModeP2G, P, n_dev, classes.ptr, g[1], g[0], sp0, dev_obstacles.ptr, dev_planes.ptr,
-                                reactions.ptr, status.ptr, cta_cache.ptr, stream);
-                tock(0);
-                for (uint32_t k = 0; k < seg; ++k) {
-                    const GridTable &gc = g[k & 1], &gn = g[(k + 1) & 1];
-                    const SimParams spk = substep_params(sp, static_cast<int>(k), apply_force && k == 0);
+                    GridTable g[2];
+                    grid_views(g, bs);
+                    const ParticleSoA P = pbuf[resort ? cur ^ 1 : cur].view(force.ptr, std::max<size_t>(world.n, 1));
                     tick(0);
-                    launch_grid_update(gc, gn, spk, dev_obstacles.ptr, dev_planes.ptr, reactions.ptr, status.ptr,
-                                       stream);
-                    tock(1);
-                    const bool last = k + 1 == seg;
-                    tick(0);
-                    launch_transfer(last ? kModeG2P : kModeG2P2G, P, n_dev, classes.ptr, gc, gn, spk,
-                                    dev_obstacles.ptr, dev_planes.ptr, reactions.ptr, status.ptr, cta_cache.ptr,
-                                    stream, &fj);
-                    tock(last ? 3 : 2);
-                    if (apply_force && k == 0) cudaMemsetAsync(force.ptr, 0, sizeof(float) * force.count, stream);
-                }
+                    launch_clear_table(g[0], g[1], bs, stream);
+                    const SimParams sp0 = substep_params(sp, -1, false);
+                    open_defer_lists(sp0);
+                    launch_transfer(kModeP2G, P, n_dev, classes.ptr, g[1], g[0], sp0, dev_obstacles.ptr, dev_planes.ptr,
+                                    reactions.ptr, status.ptr, cta_cache.ptr, stream);
+                    tock(0);
+                    for (uint32_t k = 0; k < seg; ++k) {
+                        const GridTable &gc = g[k & 1], &gn = g[(k + 1) & 1];
+                        const SimParams spk = substep_params(sp, static_cast<int>(k), apply_force && k == 0);
+                        tick(0);
+                        launch_grid_update(gc, gn, spk, dev_obstacles.ptr, dev_planes.ptr, reactions.ptr, status.ptr,
+                                           stream);
+                        tock(1);
+                        const bool last = k + 1 == seg;
+                        tick(0);
+                        launch_transfer(last ? kModeG2P : kModeG2P2G, P, n_dev, classes.ptr, gc, gn, spk,
+                                        dev_obstacles.ptr, dev_planes.ptr, reactions.ptr, status.ptr, cta_cache.ptr,
+                                        stream, &fj);
+                        tock(last ? 3 : 2);
+                        if (apply_force && k == 0) cudaMemsetAsync(force.ptr, 0, sizeof(float) * force.count, stream);
+                    }
                 }
                 if (tunable) tuner.end(static_cast<double>(n_dev) * seg, stream);
             }
