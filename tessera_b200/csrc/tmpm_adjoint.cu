@@ -968,11 +968,14 @@ __global__ void __launch_bounds__(T, 512 / T) k_rollout_backward(AdjParams P, Co
     auto replay_particles = [&](int sg, uint32_t j) {
         const int set = sg & 1;
         PartState q;
+        // The sweep's particles ran just before, in the same phase.  Without a
+        // tile their last shared-memory access is a read of the reduction's
+        // partials, which the reduction below writes; with one it is of the tile.
+        __syncthreads();
         if (j == 0) {
             q = load_state(B.ckpt + sg * sf, st, ic);
         } else {
             q = load_state(B.seg[set] + (j - 1) * sf, st, ic);
-            __syncthreads();  // the tile's last readers
             g2p_chunk<T>(P, valid, q, k, B.seg_gv[set] + (j - 1) * B.nodes, sh, box_r);
         }
         if (valid) store_state(B.seg[set] + j * sf, st, i, q);

@@ -1,0 +1,79 @@
+"""The direct path of the rollout's adjoint (a CTA that scatters node by node,
+without a shared-memory tile), reached as ordinary programs reach it: a loss on
+one tracked particle, which then dominates its CTA's velocity adjoints.
+
+Checked against central differences of the f64 oracle (1e-3 relative, the bar
+of the other adjoint tests) and between checkpoint intervals, which decide what
+the adjoint replays beside its sweep and must change the gradients only by the
+f32 order of the node sums: 1e-7 relative per sum, over 2 x SUBSTEPS substeps
+below 1e-5 of the largest component."""
+
+import numpy as np
+import pytest
+
+from oracle import oracle as O
+from tessera_b200 import scenes
+from tessera_b200.adjoint import Rollout
+
+pytestmark = pytest.mark.gpu
+SUBSTEPS = 12
+FD = 1e-3  # step of the differences: absolute for velocities, relative for moduli
+
+
+def stretched(parts, seed):
+    """The particles with a deformation 2 % off the identity, so that the moduli act from the first substep."""
+    rng = np.random.default_rng(seed)
+    F = np.eye(3) + rng.uniform(-0.02, 0.02, (parts.count, 3, 3))
+    parts.deformation[:] = F.transpose(0, 2, 1).reshape(parts.count, 9)
+    return parts
+
+
+def final_positions(params, parts, dt, v0, E):
+    p = parts.copy()
+    p.velocity[:] = v0
+    p.material_params[:, 0] = E
+    world = O.OracleWorld(params, p)
+    for _ in range(SUBSTEPS):
+        world.substep_fixed(dt)
+    return world.particles().position
+
+
+def check_gradients(params, parts, dt, tracked, seed):
+    """Gradients of a loss on the particles `tracked`, for several checkpoint intervals."""
+    rng = np.random.default_rng(seed)
+    n = parts.count
+    v0, E = parts.velocity.copy(), np.linspace(4e3, 6e3, n)
+    weight = np.zeros((n, 3))
+    weight[tracked] = rng.normal(size=(len(tracked), 3))
+
+    ref = None
+    for every in (SUBSTEPS, 1, 2, 5):
+        sim = Rollout(params, parts, dt, SUBSTEPS, checkpoint_every=every)
+        for _ in range(2):  # the second pass replays the captured launches
+            sim.forward(v0, E)
+            got = sim.backward(weight)
+            ref = ref or got
+            for a, b in zip(got, ref):
+                assert np.abs(a - b).max() <= 1e-5 * np.abs(b).max(), every
+        sim.close()
+
+    gv, gE = ref
+    assert np.abs(gE).max() > 0
+    for _ in range(3):
+        d, e = rng.normal(size=(n, 3)), rng.normal(size=n)
+        diff = (final_positions(params, parts, dt, v0 + FD * d, E) - final_positions(params, parts, dt, v0 - FD * d, E))
+        fd = float((diff * weight).sum() / (2 * FD))
+        assert abs(fd - float((gv * d).sum())) < 1e-3 * max(abs(fd), 0.1 * np.abs(gv).max()), fd
+        diff = (final_positions(params, parts, dt, v0, E * (1 + FD * e))
+                - final_positions(params, parts, dt, v0, E * (1 - FD * e)))
+        fd = float((diff * weight).sum() / (2 * FD))
+        assert abs(fd - float((gE * E * e).sum())) < 1e-3 * max(abs(fd), 0.1 * np.abs(gE * E).max()), fd
+
+
+@pytest.mark.parametrize("count", [129, 512])
+def test_loss_on_one_particle(count):
+    """Compact CTAs (their boxes fit the tile), one dominant particle, a fixed particle beside it."""
+    sc = scenes.adjoint_block(cells=4, substeps=SUBSTEPS)
+    parts = stretched(sc.particles.select(np.arange(count)), count)
+    parts.fixed[5] = 1
+    check_gradients(sc.params, parts, sc.dt, [count // 2], seed=count)
