@@ -629,6 +629,7 @@ __device__ __forceinline__ void g2p_back_chunk(const AdjParams &P, bool valid, V
     float z0 = 0.f, z1 = 0.f, z2 = 0.f, z3 = 0.f;
     tile_box<T>(P, valid, s.b, z0, z1, z2, z3, sh, box);
     if (box.ok) fill_tile<T>(P, box, gv, sh.tile);
+    else __syncthreads();  // every warp has read the partials before the second reduction writes them
     const TileRef tr = tile_ref(box, s, sh.tile);
     V3f velb = mk(0, 0, 0);
     M3f Cb = m3_zero();

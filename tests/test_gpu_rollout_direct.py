@@ -1,6 +1,7 @@
-"""The direct path of the rollout's adjoint (a CTA that scatters node by node,
-without a shared-memory tile), reached as ordinary programs reach it: a loss on
-one tracked particle, which then dominates its CTA's velocity adjoints.
+"""The direct path of the rollout's adjoint (a CTA that gathers or scatters node
+by node, without a shared-memory tile), reached as ordinary programs reach it: a
+loss on one tracked particle, which then dominates its CTA's velocity adjoints,
+and particles too far apart for their CTA's box to fit the tile.
 
 Checked against central differences of the f64 oracle (1e-3 relative, the bar
 of the other adjoint tests) and between checkpoint intervals, which decide what
@@ -13,6 +14,7 @@ import pytest
 
 from oracle import oracle as O
 from tessera_b200 import scenes
+from tessera_b200._abi import MAT_ELASTIC, density_particles, make_params
 from tessera_b200.adjoint import Rollout
 
 pytestmark = pytest.mark.gpu
@@ -77,3 +79,24 @@ def test_loss_on_one_particle(count):
     parts = stretched(sc.particles.select(np.arange(count)), count)
     parts.fixed[5] = 1
     check_gradients(sc.params, parts, sc.dt, [count // 2], seed=count)
+
+
+@pytest.mark.parametrize("fixed", [False, True])
+@pytest.mark.parametrize("loss", ["all", "one"])
+def test_scattered_particles(loss, fixed):
+    """Touching pairs spread over 26 x 26 cells: no CTA's box fits its tile.  Rows are
+    ordered by x first, so the last CTA's (partial, hence in order) second warp
+    holds the 32 particles of the third group, all of them fixed or none."""
+    h = 1.0 / 32
+    rng = np.random.default_rng(3)
+    groups = []
+    for count, lo, hi in ((64, 0.12, 0.35), (16, 0.45, 0.5), (16, 0.6, 0.65), (16, 0.75, 0.8)):
+        first = np.column_stack([rng.uniform(lo, hi, count), rng.uniform(0.1, 0.9, (count, 2))])
+        groups.append(np.stack([first, first + rng.uniform(-0.4 * h, 0.4 * h, first.shape)], 1).reshape(-1, 3))
+    params = make_params(h, bounds=((0, 0, 0), (1, 1, 1)))
+    parts = stretched(density_particles(np.concatenate(groups), h / 4, 1000.0, MAT_ELASTIC, (5e3, 0.3),
+                                        velocity=(0.1, 0.2, -0.3)), 4)
+    if fixed:
+        parts.fixed[160:192] = 1
+    tracked = np.arange(parts.count) if loss == "all" else [200]
+    check_gradients(params, parts, 1e-4, tracked, seed=5)
