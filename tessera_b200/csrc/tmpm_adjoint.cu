@@ -1066,7 +1066,7 @@ struct TmpmAdjoint {
     PinnedBuf staging;      // rows copied to and from the device
     DevBuf<float4> grid, gv, gvb, gmb;
     DevBuf<unsigned> bounds;  // whole-rollout kernels: NodeBounds per substep, and the barrier word
-    // one cooperative launch each (k_rollout_forward, k_rollout_backward)
+    // one cooperative launch each (k_rollout_forward, k_rollout_backward), until one is refused (replay)
     bool whole_forward = false, whole_backward = false;
     // Two buffer sets for replayed segments (segment sg uses set sg & 1): per
     // substep of the segment, its state, the grid after P2G (mass and
@@ -1099,22 +1099,41 @@ struct TmpmAdjoint {
         if (stream) cudaStreamDestroy(stream);
     }
 
-    // Capture `launch` (stream work only) into *exec once, then launch it.
+    // Capture `launch` (stream work only) into *exec; a launch that was refused
+    // is an error although the capture may have gone on without it.
     template <typename Fn>
-    cudaError_t replay(cudaGraphExec_t *exec, Fn launch) {
+    cudaError_t capture(cudaGraphExec_t *exec, Fn launch) {
+        cudaGraph_t g = nullptr;
+        cudaGetLastError();  // an error of an earlier call is not this capture's
+        cudaError_t e = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal);
+        if (e) return e;
+        launch();
+        const cudaError_t launched = cudaGetLastError();
+        e = cudaStreamEndCapture(stream, &g);
+        if (launched) e = launched;
+        if (!e) e = cudaGraphInstantiate(exec, g, 0);
+        if (g) cudaGraphDestroy(g);
+        if (e) *exec = nullptr;
+        return e;
+    }
+
+    // Launch a sweep's graph, captured on first use.  `whole`: as one cooperative
+    // launch.  The device may refuse that where the occupancy query did not say so
+    // (fewer SMs open to the process than the device has): the sweep then runs
+    // kernel by kernel, now and in later calls.
+    template <typename Whole, typename Stepwise>
+    cudaError_t replay(cudaGraphExec_t *exec, bool &whole, Whole launch_once, Stepwise launch_steps) {
         cudaError_t e;
-        if (!*exec) {
-            cudaGraph_t g = nullptr;
-            if ((e = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal))) return e;
-            launch();
-            if ((e = cudaStreamEndCapture(stream, &g))) return e;
-            e = cudaGraphInstantiate(exec, g, 0);
-            cudaGraphDestroy(g);
-            if (e) {
-                *exec = nullptr;
-                return e;
-            }
+        if (whole) {
+            e = *exec ? cudaSuccess : capture(exec, launch_once);
+            if (!e) e = cudaGraphLaunch(*exec, stream);
+            if (!e) return e;
+            cudaGetLastError();
+            if (*exec) cudaGraphExecDestroy(*exec);
+            *exec = nullptr;
+            whole = false;
         }
+        if (!*exec && (e = capture(exec, launch_steps))) return e;
         return cudaGraphLaunch(*exec, stream);
     }
 
@@ -1168,13 +1187,11 @@ struct TmpmAdjoint {
         return static_cast<size_t>(per_sm) * device_sm_count() * kRolloutThreads;
     }
 
-    // The forward sweep: `substeps` substeps from seg[0] (its first state)
-    // ping-ponging with its second state, a checkpoint every `every`.
+    // The forward sweep, kernel by kernel: `substeps` substeps from the initial
+    // state in seg[0] (its first state) ping-ponging with its second state, a
+    // checkpoint every `every`.
     void forward_sweep() {
-        if (whole_forward) {
-            launch_whole(k_rollout_forward<kRolloutThreads>);
-            return;
-        }
+        cudaMemcpyAsync(seg[0].ptr, initial.ptr, sizeof(float) * state_floats(), cudaMemcpyDeviceToDevice, stream);
         float *cur = seg[0].ptr, *nxt = seg[0].ptr + state_floats();
         for (uint32_t s = 0; s < substeps; ++s) {
             if (s % every == 0)
@@ -1223,17 +1240,17 @@ struct TmpmAdjoint {
         }
     }
 
-    // The adjoint sweep from adj[0] (the loss gradient of the final state),
+    void backward_whole() {
+        cudaMemsetAsync(gvb.ptr, 0, sizeof(float4) * nodes, stream);
+        launch_whole(k_rollout_backward<kRolloutThreads>);
+    }
+
+    // The adjoint sweep, kernel by kernel, from adj[0] (the loss gradient of the final state),
     // segment by segment from the last checkpoint back; the initial-state
     // adjoint ends in adj[substeps & 1].  Segment sg - 1 is replayed on `side`
     // while `stream` sweeps segment sg; the replay into a set waits for the
     // sweep that last read it (segment sg + 1), and each sweep for its replay.
     void backward_sweep() {
-        if (whole_backward) {
-            cudaMemsetAsync(gvb.ptr, 0, sizeof(float4) * nodes, stream);
-            launch_whole(k_rollout_backward<kRolloutThreads>);
-            return;
-        }
         int a = 0;
         const int segments = static_cast<int>((substeps + every - 1) / every);
         cudaEventRecord(ev_fork, stream);
@@ -1326,13 +1343,13 @@ struct TmpmAdjoint {
         cudaError_t e;
         if ((e = cudaMemcpyAsync(initial.ptr + 3 * n, h, sizeof(float) * 3 * n, cudaMemcpyHostToDevice, stream)) ||
             (e = cudaMemcpyAsync(E.ptr, h + 3 * n, sizeof(float) * n, cudaMemcpyHostToDevice, stream)) ||
-            (!whole_forward && (e = cudaMemcpyAsync(seg[0].ptr, initial.ptr, sizeof(float) * state_floats(),
-                                                    cudaMemcpyDeviceToDevice, stream))) ||
             (e = cudaMemsetAsync(err.ptr, 0, sizeof(uint32_t), stream)))
             return cuda_fail(e, "adjoint upload");
         // seg[0] holds two ping-pong states during the forward; the final state
         // is in the first of them after an even number of substeps
-        if ((e = replay(&fwd_exec, [&]() { forward_sweep(); }))) return cuda_fail(e, "adjoint forward");
+        if ((e = replay(&fwd_exec, whole_forward, [&]() { launch_whole(k_rollout_forward<kRolloutThreads>); },
+                        [&]() { forward_sweep(); })))
+            return cuda_fail(e, "adjoint forward");
         const float *cur = (substeps % 2 == 0) ? seg[0].ptr : seg[0].ptr + state_floats();
         if ((e = cudaMemcpyAsync(h, cur, sizeof(float) * 6 * n, cudaMemcpyDeviceToHost, stream)) ||
             (e = cudaStreamSynchronize(stream)))
@@ -1380,7 +1397,8 @@ struct TmpmAdjoint {
             return cuda_fail(e, "adjoint upload");
         // the parity of the final adj buffer: one flip per substep
         const int a = static_cast<int>(substeps & 1u);
-        if ((e = replay(&bwd_exec, [&]() { backward_sweep(); }))) return cuda_fail(e, "adjoint backward");
+        if ((e = replay(&bwd_exec, whole_backward, [&]() { backward_whole(); }, [&]() { backward_sweep(); })))
+            return cuda_fail(e, "adjoint backward");
         float *const vb = h, *const eb = h + 3 * n;
         if ((e = cudaMemcpyAsync(vb, adj[a].ptr + 3 * n, sizeof(float) * 3 * n, cudaMemcpyDeviceToHost, stream)) ||
             (e = cudaMemcpyAsync(eb, Ebar.ptr, sizeof(float) * n, cudaMemcpyDeviceToHost, stream)) ||

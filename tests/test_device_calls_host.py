@@ -1,0 +1,83 @@
+"""CPU tests of what the library asks of the device: its host code runs against a
+fake CUDA runtime (tests/native/fake_cudart.cpp: device memory on the heap, no
+kernel runs, every operation logged with its stream), linked with the library's
+own objects, in a process of its own."""
+
+import os
+import shutil
+import subprocess
+import sys
+
+import pytest
+
+from tessera_b200 import _native
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+OBJECTS = os.path.join(ROOT, "_build", "tmpm")
+SOURCES = os.path.join(ROOT, "tessera_b200", "csrc")
+
+PRELUDE = """
+import ctypes as C, sys
+import numpy as np
+sys.path.insert(0, {root!r})
+from tessera_b200 import _native, scenes
+_native.LIB_PATH = {lib!r}
+L = _native.lib()
+L.fake_log.restype = C.c_char_p
+L.fake_memory.argtypes = [C.c_void_p, C.c_size_t, C.c_int]
+
+def log():
+    lines = L.fake_log().decode().splitlines()
+    L.fake_clear_log()
+    return lines
+
+def count(lines, *words):
+    return sum(all(w in line for w in words) for line in lines)
+"""
+
+
+@pytest.fixture(scope="module")
+def run(tmp_path_factory):
+    if shutil.which("nvcc") is None or shutil.which("g++") is None:
+        pytest.skip("nvcc or g++ not available")
+    _native.build()  # the objects, where they are not up to date
+    lib = str(tmp_path_factory.mktemp("fake") / "libtmpm_fake.so")
+    include = os.path.join(os.path.dirname(os.path.dirname(shutil.which("nvcc"))), "include")
+    objects = sorted(os.path.join(OBJECTS, f[:-3] + ".o") for f in os.listdir(SOURCES) if f.endswith(".cu"))
+    subprocess.run(["g++", "-std=c++17", "-O1", "-fPIC", "-shared", "-I", include, "-o", lib,
+                    os.path.join(HERE, "native", "fake_cudart.cpp"), *objects, "-lpthread", "-Wl,-z,defs"],
+                   check=True, timeout=600)
+
+    def run(body):
+        r = subprocess.run([sys.executable, "-c", PRELUDE.format(root=ROOT, lib=lib) + body], capture_output=True,
+                           text=True, timeout=300, cwd=ROOT)
+        assert r.returncode == 0, r.stdout + r.stderr
+
+    return run
+
+
+@pytest.mark.parametrize("refuse", [0, 1, 2, 3])
+def test_rollout_whose_cooperative_launch_is_refused_runs_kernel_by_kernel(run, refuse):
+    """Refused when issued (1; 3: which also ends the capture) or when its graph
+    is launched (2), a whole-rollout launch must not be answered with whatever
+    the result buffers held: the sweep runs kernel by kernel, then and later."""
+    run(f"""
+from tessera_b200.adjoint import Rollout
+sc = scenes.adjoint_block(cells=2, substeps=4)
+sim = Rollout(sc.params, sc.particles, sc.dt, 4, checkpoint_every=3)
+L.fake_refuse_cooperative({refuse})
+for call in range(2):
+    log()
+    x, v = sim.forward(sc.particles.velocity, np.full(sc.particles.count, 5e3))
+    done = log()
+    whole = 0 if {refuse} else 1
+    assert count(done, "cooperative", "k_rollout_forward") == whole, done
+    assert count(done, "kernel", "k_p2g") == (0 if whole else 4), done
+    if not whole:
+        assert np.allclose(x, sc.particles.position)  # after an even count, the buffer that began as the initial state (no kernel ran)
+    sim.backward(np.ones((sc.particles.count, 3)))
+    done = log()
+    assert count(done, "cooperative", "k_rollout_backward") == whole, done
+    assert count(done, "kernel", "k_p2g_back") == (0 if whole else 4), done
+""")
