@@ -71,15 +71,17 @@ CUcontext current_context() {
     return ctx;
 }
 
-// Whether a kernel may write 32-bit words at `p`: device memory, aligned.
-bool device_words(const uint32_t *p) {
+// Whether a kernel on device `dev` may write 32-bit words at `p`: memory of
+// that device, aligned.  Another device's memory is left to copies, which reach it
+// without peer access.
+bool device_words(const uint32_t *p, int dev) {
     cudaPointerAttributes a{};
     if (reinterpret_cast<uintptr_t>(p) % sizeof(uint32_t) != 0) return false;
     if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    return a.type == cudaMemoryTypeDevice;
+    return a.type == cudaMemoryTypeDevice && a.device == dev;
 }
 
 }  // namespace
@@ -147,9 +149,9 @@ extern "C" TmpmStatus tmpm_sort_by_block_noalloc(const float *positions, size_t 
     // by the key kernel), so nothing has to start at zero.
     const int n = static_cast<int>(count);
     const tmpm::BinSource src{positions, stride, n, 1.0f / h32, nullptr, nullptr, nullptr};
-    // The last pass writes device buffers itself; anything else (a buffer that
-    // only a copy can reach, or one not aligned to its words) gets a copy.
-    const bool direct = device_words(order_out) && (!keys_out || device_words(keys_out));
+    // The last pass writes this device's buffers itself; anything else (a buffer
+    // that only a copy can reach, or one not aligned to its words) gets a copy.
+    const bool direct = device_words(order_out, dev) && (!keys_out || device_words(keys_out, dev));
     const int r = tmpm::bin_and_sort(src, sb, tmpm::kSortBitsScene, direct ? keys_out : nullptr,
                                      direct ? order_out : nullptr, s);
     e = cudaGetLastError();  // launch errors of the binning and radix kernels

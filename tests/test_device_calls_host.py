@@ -81,3 +81,28 @@ for call in range(2):
     assert count(done, "cooperative", "k_rollout_backward") == whole, done
     assert count(done, "kernel", "k_p2g_back") == (0 if whole else 4), done
 """)
+
+
+@pytest.mark.parametrize("device", [0, 1])
+@pytest.mark.parametrize("with_keys", [False, True])
+@pytest.mark.parametrize("offset", [0, 2])
+def test_binning_writes_only_words_of_its_own_device(run, device, with_keys, offset):
+    """The last pass stores to the caller's buffers itself only where a kernel may:
+    aligned memory of the current device.  Another device's memory is reached by
+    copies, which need no peer access."""
+    run(f"""
+n = 300
+pos = np.random.default_rng(1).uniform(0, 1, (3, n)).astype(np.float32)
+own, out = np.zeros(n + 1, np.uint32), np.zeros(n + 1, np.uint32)
+L.fake_memory(pos.ctypes.data, pos.nbytes, 0)
+L.fake_memory(own.ctypes.data, own.nbytes, 0)
+L.fake_memory(out.ctypes.data, out.nbytes, {device})
+order, keys = (own.ctypes.data, out.ctypes.data + {offset}) if {with_keys} else (out.ctypes.data + {offset}, None)
+assert L.tmpm_sort_by_block_noalloc(pos.ctypes.data, n, n, 1 / 64, order, keys, None) == 0, L.tmpm_last_error()
+done = log()
+assert count(done, "kernel", "k_small_pass") == 3
+direct = {device} == 0 and {offset} == 0
+assert count(done, "copy kind=3", "dst=%#x " % order) == (0 if direct else 1), done
+if keys:
+    assert count(done, "copy kind=3", "dst=%#x " % keys) == (0 if direct else 1), done
+""")
