@@ -357,7 +357,7 @@ struct TmpmBatch {
         const size_t nodes = std::max(grow.nodes, need.nodes);
         cudaError_t e;
         for (int g = 0; g < 2; ++g)
-            if ((e = grids[g].alloc(static_cast<uint32_t>(std::max(grow.blocks, need.blocks)), nodes)))
+            if ((e = grids[g].alloc(static_cast<uint32_t>(std::max(grow.blocks, need.blocks)), nodes, stream)))
                 return cuda_fail(e, "cudaMalloc grid");
         ++epoch;
         return TMPM_OK;

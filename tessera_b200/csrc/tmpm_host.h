@@ -714,7 +714,9 @@ struct GridBuffers {
     DevBuf<int4> coords;
     uint32_t capacity = 0, max_blocks = 0;
     size_t pool_nodes = 0;
-    cudaError_t alloc(uint32_t blocks, size_t nodes = 0) {
+    // `stream`: the owner's, whose kernels are the first to read the table's words
+    // (no legacy-stream copy is ordered before a non-blocking stream's work).
+    cudaError_t alloc(uint32_t blocks, size_t nodes, cudaStream_t stream) {
         nodes = std::max(nodes, static_cast<size_t>(blocks) * kNodesPerBlock);
         uint32_t cap = 1024;
         while (cap < 2u * blocks) cap <<= 1;
@@ -722,8 +724,9 @@ struct GridBuffers {
         if ((e = keys.alloc(cap)) || (e = vals.alloc(cap)) || (e = count.alloc(kTableWords)) || (e = pool.alloc(nodes)) ||
             (e = coords.alloc(blocks)))
             return e;
-        const uint32_t words[kTableWords] = {0, ~0u, 0, 0};
-        if ((e = cudaMemcpy(count.ptr, words, sizeof words, cudaMemcpyHostToDevice))) return e;
+        if ((e = cudaMemsetAsync(count.ptr, 0, sizeof(uint32_t) * kTableWords, stream)) ||
+            (e = cudaMemsetAsync(count.ptr + kDirtyWord, 0xFF, sizeof(uint32_t), stream)))
+            return e;
         capacity = cap;
         max_blocks = blocks;
         pool_nodes = nodes;

@@ -326,7 +326,7 @@ struct TmpmSession {
         if (force_dirty) cudaMemsetAsync(force.ptr, 0, sizeof(float) * force.count, stream);
         for (int g = 0; g < 2; ++g)
             if (grids[g].max_blocks != plan.blocks || grids[g].pool_nodes != plan.nodes)
-                if ((e = grids[g].alloc(static_cast<uint32_t>(plan.blocks), plan.nodes))) return cuda_fail(e, "cudaMalloc grid");
+                if ((e = grids[g].alloc(static_cast<uint32_t>(plan.blocks), plan.nodes, stream))) return cuda_fail(e, "cudaMalloc grid");
         size_t sort_cap = pbuf[0].cap;
         if (sort_keys[0].count < sort_cap) {
             for (int b = 0; b < 2; ++b)

@@ -106,3 +106,33 @@ assert count(done, "copy kind=3", "dst=%#x " % order) == (0 if direct else 1), d
 if keys:
     assert count(done, "copy kind=3", "dst=%#x " % keys) == (0 if direct else 1), done
 """)
+
+
+# the words after each grid table's block count (two tables): cleared, then one set
+# to ~0, on the stream of the segment that reads them, before it
+TABLE_WORDS = """
+    lines = log()
+    first = next(i for i, line in enumerate(lines) if "k_segment" in line)
+    stream = lines[first].split("stream=")[1]
+    assert stream != "(nil)"
+    cleared = [line.split("dst=")[1].split()[0] for line in lines[:first]
+               if line.startswith("set") and "bytes=16 " in line and line.endswith("stream=" + stream)]
+    marked = ["set dst=%#x bytes=4 stream=%s" % (int(p, 16) + 4, stream) for p in cleared]
+    assert sum(m in lines[:first] for m in marked) == 2, lines[:first]
+"""
+
+
+def test_table_words_are_set_on_the_stream_that_reads_them(run):
+    run("""
+def check():
+""" + TABLE_WORDS + """
+from tessera_b200.batch import Batch
+from tessera_b200.session import Session
+sc = scenes.batch_scene(3, cells=4)
+s = Session(sc.params, sc.particles, sc.dt)
+s.submit_steps(3)
+check()
+b = Batch()
+b.run({b.add_scene(sc.params, sc.particles, sc.dt): 3})
+check()
+""")
