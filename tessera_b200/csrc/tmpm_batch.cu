@@ -363,7 +363,7 @@ struct TmpmBatch {
         return TMPM_OK;
     }
 
-    // Idle only (synchronous copy from the host table).
+    // Idle only.  On the stream whose kernels read the table, as every upload.
     TmpmStatus upload_classes() {
         if (classes.table.size() == classes_uploaded) return TMPM_OK;
         cudaError_t e;
@@ -371,8 +371,9 @@ struct TmpmBatch {
             if ((e = dclasses.alloc(std::max<size_t>(2 * classes.table.size(), 64)))) return cuda_fail(e, "cudaMalloc classes");
             ++epoch;
         }
-        if ((e = cudaMemcpy(dclasses.ptr, classes.table.data(), sizeof(DevClass) * classes.table.size(),
-                            cudaMemcpyHostToDevice)))
+        if ((e = cudaMemcpyAsync(dclasses.ptr, classes.table.data(), sizeof(DevClass) * classes.table.size(),
+                                 cudaMemcpyHostToDevice, stream)) ||
+            (e = cudaStreamSynchronize(stream)))
             return cuda_fail(e, "upload classes");
         classes_uploaded = classes.table.size();
         ++epoch;  // the transfer variant (plastic or not) captured in a graph follows the class table

@@ -1324,10 +1324,11 @@ TmpmStatus tmpm_rigid_attach(TmpmSession *s, const TmpmRigidBody *bodies, size_t
     if ((e = s->rigid_bodies.alloc(std::max<size_t>(body_count, 1))) ||
         (e = s->rigid_maps.alloc(std::max<size_t>(mapping_count, 1))))
         return s->cuda_fail(e, "cudaMalloc rigid");
-    if ((body_count && (e = cudaMemcpy(s->rigid_bodies.ptr, db.data(), sizeof(DevRigid) * body_count,
-                                       cudaMemcpyHostToDevice))) ||
-        (mapping_count && (e = cudaMemcpy(s->rigid_maps.ptr, dm.data(), sizeof(DevRigidMap) * mapping_count,
-                                          cudaMemcpyHostToDevice))))
+    if ((body_count && (e = cudaMemcpyAsync(s->rigid_bodies.ptr, db.data(), sizeof(DevRigid) * body_count,
+                                            cudaMemcpyHostToDevice, s->stream))) ||
+        (mapping_count && (e = cudaMemcpyAsync(s->rigid_maps.ptr, dm.data(), sizeof(DevRigidMap) * mapping_count,
+                                               cudaMemcpyHostToDevice, s->stream))) ||
+        (e = cudaStreamSynchronize(s->stream)))
         return s->cuda_fail(e, "rigid upload");
     s->rigid_body_count = body_count;
     s->rigid_map_count = mapping_count;

@@ -136,3 +136,25 @@ b = Batch()
 b.run({b.add_scene(sc.params, sc.particles, sc.dt): 3})
 check()
 """)
+
+
+def test_uploads_are_ordered_before_the_kernels_that_read_them(run):
+    """No host-to-device copy on the legacy stream: from pageable memory it may
+    return before its data has arrived, and non-blocking streams do not wait for it."""
+    run("""
+from tessera_b200._abi import Obstacle, TmpmRigidBody, TmpmRigidMapping
+from tessera_b200.batch import Batch
+from tessera_b200.session import Session
+sc = scenes.batch_scene(3, cells=4)
+s = Session(sc.params, sc.particles, sc.dt, obstacles=[Obstacle.sphere((0.5, 0.5, 0.9), 0.05)])
+s.rigid_attach([TmpmRigidBody.make((0.5, 0.5, 0.9), 2.0, inverse_inertia=(5.0, 5.0, 5.0))], [TmpmRigidMapping.make(0)])
+s.rigid_step(2)
+b = Batch()
+b.run({b.add_scene(sc.params, sc.particles, sc.dt): 3})
+from tessera_b200.adjoint import Rollout
+sc = scenes.adjoint_block(cells=2, substeps=4)
+Rollout(sc.params, sc.particles, sc.dt, 4).forward()
+lines = log()
+assert count(lines, "copy kind=1") > 10
+assert count(lines, "copy kind=1", "stream=(nil)") == 0, [l for l in lines if "(nil)" in l]
+""")
