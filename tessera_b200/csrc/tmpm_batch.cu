@@ -196,6 +196,7 @@ struct TmpmBatch {
     double last_ms = 0.0;
     LaunchTuner tuner;  // transfer launch configuration (tuned on the first batches unless fixed)
     bool big_blocks_ok = false;  // the node pools hold the live scenes in 8^3 blocks too
+    bool whole_segments = true;  // small batches as one cooperative launch, until one is refused (enqueue)
 
     struct GraphKey {
         uint32_t steps;
@@ -635,7 +636,8 @@ struct TmpmBatch {
         const int n = static_cast<int>(n_live);
         SimParams sp0 = sp;
         sp0.step_index = -1;
-        if (launch_small_segment(dst, n, dclasses.ptr, g[1], g[0], sp0, nullptr, nullptr, nullptr, status.ptr,
+        if (whole_segments &&
+            launch_small_segment(dst, n, dclasses.ptr, g[1], g[0], sp0, nullptr, nullptr, nullptr, status.ptr,
                                  cta_cache.ptr, static_cast<int>(steps), stream))
             return;
         launch_clear_table(g[0], g[1], bs, stream);
@@ -660,6 +662,33 @@ struct TmpmBatch {
         }
     }
 
+    // The batch's kernels replayed from their captured graph (captured now if
+    // new); `timed` opens the tuner's trial, once; `what`: the call that failed.
+    cudaError_t replay_batch(uint32_t steps, int config, bool &timed, const char *&what) {
+        GraphKey key{steps, n_phys, n_live, cur, epoch, config};
+        cudaError_t e;
+        auto it = graphs.find(key);
+        if (it == graphs.end()) {
+            if (graphs.size() > 16) drop_graphs();
+            cudaGraph_t graph = nullptr;
+            what = "cudaStreamBeginCapture";
+            if ((e = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal))) return e;
+            launch_batch(steps, config);
+            what = "cudaStreamEndCapture";
+            if ((e = cudaStreamEndCapture(stream, &graph))) return e;
+            cudaGraphExec_t exec = nullptr;
+            e = cudaGraphInstantiate(&exec, graph, 0);
+            cudaGraphDestroy(graph);
+            what = "cudaGraphInstantiate";
+            if (e) return e;
+            it = graphs.emplace(key, exec).first;
+        }
+        if (timed) tuner.begin(config, stream);
+        timed = false;
+        what = "cudaGraphLaunch";
+        return cudaGraphLaunch(it->second, stream);
+    }
+
     TmpmStatus enqueue(uint32_t steps) {
         cudaError_t e;
         TmpmStatus st;
@@ -675,23 +704,16 @@ struct TmpmBatch {
             const int config = tunable ? tuner.config(big_blocks_ok, true) : 0;
             const double work = static_cast<double>(n_live) * steps;
             if (options.use_graphs) {
-                GraphKey key{steps, n_phys, n_live, cur, epoch, config};
-                auto it = graphs.find(key);
-                if (it == graphs.end()) {
-                    if (graphs.size() > 16) drop_graphs();
-                    cudaGraph_t graph = nullptr;
-                    if ((e = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal)))
-                        return cuda_fail(e, "cudaStreamBeginCapture");
-                    launch_batch(steps, config);
-                    if ((e = cudaStreamEndCapture(stream, &graph))) return cuda_fail(e, "cudaStreamEndCapture");
-                    cudaGraphExec_t exec = nullptr;
-                    e = cudaGraphInstantiate(&exec, graph, 0);
-                    cudaGraphDestroy(graph);
-                    if (e) return cuda_fail(e, "cudaGraphInstantiate");
-                    it = graphs.emplace(key, exec).first;
+                const char *what = "";
+                bool timed = tunable;
+                e = replay_batch(steps, config, timed, what);
+                if (e && whole_segments) {  // a cooperative launch was refused, as in a session
+                    cudaGetLastError();
+                    drop_graphs();
+                    whole_segments = false;
+                    e = replay_batch(steps, config, timed, what);
                 }
-                if (tunable) tuner.begin(config, stream);
-                if ((e = cudaGraphLaunch(it->second, stream))) return cuda_fail(e, "cudaGraphLaunch");
+                if (e) return cuda_fail(e, what);
             } else {
                 if (tunable) tuner.begin(config, stream);
                 launch_batch(steps, config);

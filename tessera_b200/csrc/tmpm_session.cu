@@ -124,6 +124,7 @@ struct TmpmSession {
     std::map<std::string, cudaGraphExec_t> seg_graphs;
     int stored_shape = -1;   // launch shape whose per-CTA interleave the device rows hold
     bool big_blocks_ok = false;  // the node pools hold the scene in 8^3 blocks too
+    bool whole_segments = true;  // small segments as one cooperative launch, until one is refused (run_segment_graph)
 
     ~TmpmSession() {
         if (stream) {
@@ -438,7 +439,8 @@ struct TmpmSession {
         GridTable g[2];
         grid_views(g, bs);
         const ParticleSoA P = pbuf[rows].view(force.ptr, std::max<size_t>(world.n, 1));
-        if (launch_small_segment(P, n_dev, classes.ptr, g[1], g[0], substep_params(sp, -1, apply_force),
+        if (whole_segments &&
+            launch_small_segment(P, n_dev, classes.ptr, g[1], g[0], substep_params(sp, -1, apply_force),
                                  dev_obstacles.ptr, dev_planes.ptr, reactions.ptr, status.ptr, cta_cache.ptr,
                                  static_cast<int>(seg), stream)) {
             if (apply_force) cudaMemsetAsync(force.ptr, 0, sizeof(float) * force.count, stream);
@@ -507,26 +509,43 @@ struct TmpmSession {
         return std::string(reinterpret_cast<const char *>(&k), sizeof k);
     }
 
-    // One segment replayed from its captured graph (captured now if new).
-    TmpmStatus run_segment_graph(const SimParams &sp, bool resort, uint32_t seg, bool apply_force) {
+    // One segment replayed from its captured graph (captured now if new); `what`: the call that failed.
+    cudaError_t replay_segment(const SimParams &sp, bool resort, uint32_t seg, bool apply_force, const char *&what) {
         const std::string key = segment_key(sp, cur, resort, seg, apply_force);
         auto it = seg_graphs.find(key);
         cudaError_t e;
         if (it == seg_graphs.end()) {
             if (seg_graphs.size() >= 16) drop_graphs();
             cudaGraph_t g = nullptr;
-            if ((e = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal)))
-                return cuda_fail(e, "cudaStreamBeginCapture");
+            what = "cudaStreamBeginCapture";
+            if ((e = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal))) return e;
             launch_segment(sp, cur, resort, seg, apply_force);
-            if ((e = cudaStreamEndCapture(stream, &g))) return cuda_fail(e, "cudaStreamEndCapture");
+            what = "cudaStreamEndCapture";
+            if ((e = cudaStreamEndCapture(stream, &g))) return e;
             cudaGraphExec_t exec = nullptr;
             e = cudaGraphInstantiate(&exec, g, 0);
             cudaGraphDestroy(g);
-            if (e) return cuda_fail(e, "cudaGraphInstantiate");
+            what = "cudaGraphInstantiate";
+            if (e) return e;
             it = seg_graphs.emplace(key, exec).first;
         }
-        if ((e = cudaGraphLaunch(it->second, stream))) return cuda_fail(e, "cudaGraphLaunch");
-        return TMPM_OK;
+        what = "cudaGraphLaunch";
+        return cudaGraphLaunch(it->second, stream);
+    }
+    // The device may refuse the cooperative launch of a small segment by ending its
+    // capture or by failing its graph, where the occupancy query did not say so
+    // (fewer SMs open to the process than the device has): the segments then
+    // run kernel by kernel, this one and later ones.
+    TmpmStatus run_segment_graph(const SimParams &sp, bool resort, uint32_t seg, bool apply_force) {
+        const char *what = "";
+        cudaError_t e = replay_segment(sp, resort, seg, apply_force, what);
+        if (e && whole_segments) {
+            cudaGetLastError();
+            drop_graphs();
+            whole_segments = false;
+            e = replay_segment(sp, resort, seg, apply_force, what);
+        }
+        return e ? cuda_fail(e, what) : TMPM_OK;
     }
 
     // Queue `steps` resident substeps on the stream (encode_prepared, gpu.rs:1729-1777).

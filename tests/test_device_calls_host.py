@@ -158,3 +158,30 @@ lines = log()
 assert count(lines, "copy kind=1") > 10
 assert count(lines, "copy kind=1", "stream=(nil)") == 0, [l for l in lines if "(nil)" in l]
 """)
+
+
+@pytest.mark.parametrize("refuse", [0, 1, 2, 3])
+def test_segment_whose_cooperative_launch_is_refused_runs_kernel_by_kernel(run, refuse):
+    """As for a rollout: captured segments of a session (16 substeps) and launched ones (2), and a batch's."""
+    run(f"""
+from tessera_b200.batch import Batch
+from tessera_b200.session import Session
+sc = scenes.batch_scene(3, cells=4)
+L.fake_refuse_cooperative({refuse})
+s = Session(sc.params, sc.particles, sc.dt, launch_shape=0)
+b = Batch(launch_shape=0)
+scene = b.add_scene(sc.params, sc.particles, sc.dt)
+log()
+for steps in (16, 2, 16):
+    for call in (lambda: s.step(steps), lambda: b.run({{scene: steps}})):
+        call()
+        done = log()
+        # refused only when a graph is launched, a segment without one still goes whole at first
+        if {refuse} == 0:
+            assert count(done, "cooperative", "k_segment") == 1, done
+            assert count(done, "kernel", "k_grid") == 0, done
+        else:
+            assert count(done, "cooperative", "k_segment") == 0, done
+            assert count(done, "kernel", "k_grid") == steps, done
+assert s.substeps() == 34 and b.substeps(scene) == 34
+""")
