@@ -268,6 +268,10 @@ extern "C" {
                               key_out: *mut u32) -> TmpmStatus;
     pub fn tmpm_debug_p2g(session: *mut TmpmSession, cells_out: *mut i32, mass_momentum_out: *mut f32,
                           capacity: usize, count: *mut usize) -> TmpmStatus;
+    pub fn tmpm_debug_session_segments(session: *const TmpmSession, whole: *mut u64, stepwise: *mut u64);
+    pub fn tmpm_debug_batch_segments(batch: *const TmpmBatch, whole: *mut u64, stepwise: *mut u64);
+    pub fn tmpm_debug_rollout_whole(adjoint: *const TmpmAdjoint) -> i32;
+    pub fn tmpm_debug_rollout_stepwise(adjoint: *mut TmpmAdjoint);
     pub fn tmpm_bench_substeps(session: *mut TmpmSession, steps: u32, ms: *mut f64, kernel_ms: *mut f64,
                                kernel_count: usize) -> TmpmStatus;
 

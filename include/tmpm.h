@@ -470,12 +470,26 @@ TmpmStatus tmpm_debug_binning(TmpmSession *session, uint32_t *world_index_out,
 TmpmStatus tmpm_debug_p2g(TmpmSession *session, int32_t *cells_out, float *mass_momentum_out,
                           size_t capacity, size_t *count);
 
+/* How segments were launched so far (test hook): *whole as one cooperative launch
+ * (small scenes), *stepwise kernel by kernel.  A segment replayed from a graph
+ * counts when it was captured. */
+void tmpm_debug_session_segments(const TmpmSession *session, uint64_t *whole, uint64_t *stepwise);
+void tmpm_debug_batch_segments(const TmpmBatch *batch, uint64_t *whole, uint64_t *stepwise);
+
+/* Which sweeps of a rollout are one cooperative launch (test hook): bit 0 the
+ * forward, bit 1 the adjoint; and a rollout's sweeps kernel by kernel from its
+ * next call on. */
+int32_t tmpm_debug_rollout_whole(const TmpmAdjoint *adjoint);
+void tmpm_debug_rollout_stepwise(TmpmAdjoint *adjoint);
+
 /* Kernel timing (bench hook): time `steps` substeps of the resident path on the
  * session stream with CUDA events; returns milliseconds via *ms (host waits
  * between submissions included).  The substeps go in submissions of at most 64,
  * each waited for before the next, as a caller stepping frame by frame runs
  * them.  Per-kernel averages (ms per launch) go to kernel_ms[0..n) in the order
- * p2g, grid, g2p2g, g2p, resort when kernel_ms is non-NULL. */
+ * p2g, grid, g2p2g, g2p, resort when kernel_ms is non-NULL; the substeps then
+ * always run kernel by kernel, also where a small scene's segments are otherwise
+ * one launch, whose share of these kernels the averages are not. */
 TmpmStatus tmpm_bench_substeps(TmpmSession *session, uint32_t steps, double *ms,
                                double *kernel_ms, size_t kernel_count);
 

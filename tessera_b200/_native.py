@@ -87,6 +87,13 @@ def lib():
     L.tmpm_debug_binning.restype = S
     L.tmpm_debug_p2g.argtypes = [P, P, P, C.c_size_t, C.POINTER(C.c_size_t)]
     L.tmpm_debug_p2g.restype = S
+    for name in ("tmpm_debug_session_segments", "tmpm_debug_batch_segments"):
+        getattr(L, name).argtypes = [P, C.POINTER(C.c_uint64), C.POINTER(C.c_uint64)]
+        getattr(L, name).restype = None
+    L.tmpm_debug_rollout_whole.argtypes = [P]
+    L.tmpm_debug_rollout_whole.restype = C.c_int32
+    L.tmpm_debug_rollout_stepwise.argtypes = [P]
+    L.tmpm_debug_rollout_stepwise.restype = None
     L.tmpm_bench_substeps.argtypes = [P, C.c_uint32, C.POINTER(C.c_double), P, C.c_size_t]
     L.tmpm_bench_substeps.restype = S
     L.tmpm_sort_by_block_noalloc.argtypes = [P, C.c_size_t, C.c_size_t, C.c_double, P, P, P]
@@ -182,6 +189,13 @@ def launch_shapes() -> list[tuple[int, int, int]]:
             raise RuntimeError(f"launch shape {k}: {L.tmpm_last_error().decode()}")
         out.append((int(t.value), int(b.value), int(e.value)))
     return out
+
+
+def segment_launches(fn, handle) -> tuple[int, int]:
+    """Segments of a session or batch launched (whole, kernel by kernel) so far."""
+    whole, stepwise = C.c_uint64(0), C.c_uint64(0)
+    fn(handle, C.byref(whole), C.byref(stepwise))
+    return int(whole.value), int(stepwise.value)
 
 
 def query_launch_shape(fn, handle) -> dict:

@@ -1666,6 +1666,20 @@ TmpmStatus tmpm_adjoint_backward(TmpmAdjoint *a, const double *position_grad, co
     return a->backward(position_grad, velocity_grad, velocity0_grad, young_grad);
 }
 
+int32_t tmpm_debug_rollout_whole(const TmpmAdjoint *a) {
+    return a ? (a->whole_forward ? 1 : 0) | (a->whole_backward ? 2 : 0) : 0;
+}
+
+void tmpm_debug_rollout_stepwise(TmpmAdjoint *a) {
+    if (!a) return;
+    cudaSetDevice(a->device);
+    cudaStreamSynchronize(a->stream);
+    if (a->fwd_exec) cudaGraphExecDestroy(a->fwd_exec);
+    if (a->bwd_exec) cudaGraphExecDestroy(a->bwd_exec);
+    a->fwd_exec = a->bwd_exec = nullptr;
+    a->whole_forward = a->whole_backward = false;
+}
+
 const char *tmpm_adjoint_last_error_message(const TmpmAdjoint *a) {
     return a ? a->last_error.c_str() : g_last_error.c_str();
 }

@@ -196,6 +196,7 @@ struct TmpmBatch {
     double last_ms = 0.0;
     LaunchTuner tuner;  // transfer launch configuration (tuned on the first batches unless fixed)
     bool big_blocks_ok = false;  // the node pools hold the live scenes in 8^3 blocks too
+    uint64_t whole_launches = 0, stepwise_launches = 0;  // batches issued or captured (tmpm_debug_batch_segments)
     bool whole_segments = true;  // small batches as one cooperative launch, until one is refused (enqueue)
 
     struct GraphKey {
@@ -638,8 +639,11 @@ struct TmpmBatch {
         sp0.step_index = -1;
         if (whole_segments &&
             launch_small_segment(dst, n, dclasses.ptr, g[1], g[0], sp0, nullptr, nullptr, nullptr, status.ptr,
-                                 cta_cache.ptr, static_cast<int>(steps), stream))
+                                 cta_cache.ptr, static_cast<int>(steps), stream)) {
+            ++whole_launches;
             return;
+        }
+        ++stepwise_launches;
         launch_clear_table(g[0], g[1], bs, stream);
         // the fused transfer's deferred-chunk lists (as in a session): emptied
         // before the opening P2G, then by each grid update for its transfer
@@ -1279,6 +1283,11 @@ TmpmStatus tmpm_batch_read_scene(TmpmBatch *b, uint32_t scene, TmpmParticleArray
     if (st != TMPM_OK) return b->fail(st, s->error.empty() ? b->last_error : s->error);
     s->world.store(*out);
     return TMPM_OK;
+}
+
+void tmpm_debug_batch_segments(const TmpmBatch *b, uint64_t *whole, uint64_t *stepwise) {
+    if (whole) *whole = b ? b->whole_launches : 0;
+    if (stepwise) *stepwise = b ? b->stepwise_launches : 0;
 }
 
 double tmpm_batch_last_ms(const TmpmBatch *b) { return b ? b->last_ms : 0.0; }

@@ -124,6 +124,7 @@ struct TmpmSession {
     std::map<std::string, cudaGraphExec_t> seg_graphs;
     int stored_shape = -1;   // launch shape whose per-CTA interleave the device rows hold
     bool big_blocks_ok = false;  // the node pools hold the scene in 8^3 blocks too
+    uint64_t whole_launches = 0, stepwise_launches = 0;  // segments issued or captured (tmpm_debug_session_segments)
     bool whole_segments = true;  // small segments as one cooperative launch, until one is refused (run_segment_graph)
 
     ~TmpmSession() {
@@ -435,28 +436,46 @@ struct TmpmSession {
     // The table clear, P2G and substeps of a segment on row buffer `rows`: one
     // launch for a small scene, otherwise kernel by kernel.
     void launch_steps(const SimParams &sp, int rows, uint32_t seg, bool apply_force) {
-        const int bs = sp.block_shift;
         GridTable g[2];
-        grid_views(g, bs);
+        grid_views(g, sp.block_shift);
         const ParticleSoA P = pbuf[rows].view(force.ptr, std::max<size_t>(world.n, 1));
         if (whole_segments &&
             launch_small_segment(P, n_dev, classes.ptr, g[1], g[0], substep_params(sp, -1, apply_force),
                                  dev_obstacles.ptr, dev_planes.ptr, reactions.ptr, status.ptr, cta_cache.ptr,
                                  static_cast<int>(seg), stream)) {
             if (apply_force) cudaMemsetAsync(force.ptr, 0, sizeof(float) * force.count, stream);
+            ++whole_launches;
             return;
         }
-        launch_clear_table(g[0], g[1], bs, stream);
-        const SimParams sp0 = substep_params(sp, -1, false);
-        open_defer_lists(sp0);
-        launch_transfer(kModeP2G, P, n_dev, classes.ptr, g[1], g[0], sp0, dev_obstacles.ptr, dev_planes.ptr,
-                        reactions.ptr, status.ptr, cta_cache.ptr, stream);
+        launch_kernels(sp, rows, seg, apply_force, [](int, auto launch) { launch(); });
+    }
+
+    // The same kernel by kernel.  Each launch goes through timed(slot, launch), the
+    // slot as in tmpm_bench_substeps: 0 clear and P2G, 1 grid, 2 fused transfer, 3 G2P.
+    template <typename Timed>
+    void launch_kernels(const SimParams &sp, int rows, uint32_t seg, bool apply_force, Timed timed) {
+        GridTable g[2];
+        grid_views(g, sp.block_shift);
+        const ParticleSoA P = pbuf[rows].view(force.ptr, std::max<size_t>(world.n, 1));
+        ++stepwise_launches;
+        timed(0, [&]() {
+            launch_clear_table(g[0], g[1], sp.block_shift, stream);
+            const SimParams sp0 = substep_params(sp, -1, false);
+            open_defer_lists(sp0);
+            launch_transfer(kModeP2G, P, n_dev, classes.ptr, g[1], g[0], sp0, dev_obstacles.ptr, dev_planes.ptr,
+                            reactions.ptr, status.ptr, cta_cache.ptr, stream);
+        });
         for (uint32_t k = 0; k < seg; ++k) {
             const GridTable &gc = g[k & 1], &gn = g[(k + 1) & 1];
             const SimParams spk = substep_params(sp, static_cast<int>(k), apply_force && k == 0);
-            launch_grid_update(gc, gn, spk, dev_obstacles.ptr, dev_planes.ptr, reactions.ptr, status.ptr, stream);
-            launch_transfer(k + 1 == seg ? kModeG2P : kModeG2P2G, P, n_dev, classes.ptr, gc, gn, spk,
-                            dev_obstacles.ptr, dev_planes.ptr, reactions.ptr, status.ptr, cta_cache.ptr, stream, &fj);
+            timed(1, [&]() {
+                launch_grid_update(gc, gn, spk, dev_obstacles.ptr, dev_planes.ptr, reactions.ptr, status.ptr, stream);
+            });
+            const bool last = k + 1 == seg;
+            timed(last ? 3 : 2, [&]() {
+                launch_transfer(last ? kModeG2P : kModeG2P2G, P, n_dev, classes.ptr, gc, gn, spk, dev_obstacles.ptr,
+                                dev_planes.ptr, reactions.ptr, status.ptr, cta_cache.ptr, stream, &fj);
+            });
             if (apply_force && k == 0) cudaMemsetAsync(force.ptr, 0, sizeof(float) * force.count, stream);
         }
     }
@@ -612,7 +631,7 @@ struct TmpmSession {
                     st = run_segment_graph(sp, resort, seg, apply_force);
                 if (probe) tuner.probe_end(static_cast<double>(n_dev) * seg, stream);
             } else {
-                // launch_segment's kernels one by one, timed with `kernel_ms`
+                // launched directly; with `kernel_ms` always kernel by kernel, each timed
                 if (resort) {
                     tick(0);
                     ParticleSoA src = soa();
@@ -622,35 +641,15 @@ struct TmpmSession {
                     tock(4);
                 }
                 if (tunable) tuner.begin(config, stream);
-                if (!kernel_ms) {
-                    launch_steps(sp, resort ? cur ^ 1 : cur, seg, apply_force);
-                } else {
-                    GridTable g[2];
-                    grid_views(g, bs);
-                    const ParticleSoA P = pbuf[resort ? cur ^ 1 : cur].view(force.ptr, std::max<size_t>(world.n, 1));
-                    tick(0);
-                    launch_clear_table(g[0], g[1], bs, stream);
-                    const SimParams sp0 = substep_params(sp, -1, false);
-                    open_defer_lists(sp0);
-                    launch_transfer(kModeP2G, P, n_dev, classes.ptr, g[1], g[0], sp0, dev_obstacles.ptr, dev_planes.ptr,
-                                    reactions.ptr, status.ptr, cta_cache.ptr, stream);
-                    tock(0);
-                    for (uint32_t k = 0; k < seg; ++k) {
-                        const GridTable &gc = g[k & 1], &gn = g[(k + 1) & 1];
-                        const SimParams spk = substep_params(sp, static_cast<int>(k), apply_force && k == 0);
+                const int rows = resort ? cur ^ 1 : cur;
+                if (!kernel_ms)
+                    launch_steps(sp, rows, seg, apply_force);
+                else
+                    launch_kernels(sp, rows, seg, apply_force, [&](int slot, auto launch) {
                         tick(0);
-                        launch_grid_update(gc, gn, spk, dev_obstacles.ptr, dev_planes.ptr, reactions.ptr, status.ptr,
-                                           stream);
-                        tock(1);
-                        const bool last = k + 1 == seg;
-                        tick(0);
-                        launch_transfer(last ? kModeG2P : kModeG2P2G, P, n_dev, classes.ptr, gc, gn, spk,
-                                        dev_obstacles.ptr, dev_planes.ptr, reactions.ptr, status.ptr, cta_cache.ptr,
-                                        stream, &fj);
-                        tock(last ? 3 : 2);
-                        if (apply_force && k == 0) cudaMemsetAsync(force.ptr, 0, sizeof(float) * force.count, stream);
-                    }
-                }
+                        launch();
+                        tock(slot);
+                    });
                 if (tunable) tuner.end(static_cast<double>(n_dev) * seg, stream);
             }
             if (resort) {
@@ -1222,6 +1221,11 @@ TmpmStatus tmpm_debug_p2g(TmpmSession *s, int32_t *cells_out, float *mm_out, siz
     if (mm_out && got) cudaMemcpy(mm_out, vals.ptr, sizeof(float4) * got, cudaMemcpyDeviceToHost);
     if (count) *count = total;
     return TMPM_OK;
+}
+
+void tmpm_debug_session_segments(const TmpmSession *s, uint64_t *whole, uint64_t *stepwise) {
+    if (whole) *whole = s ? s->whole_launches : 0;
+    if (stepwise) *stepwise = s ? s->stepwise_launches : 0;
 }
 
 TmpmStatus tmpm_bench_substeps(TmpmSession *s, uint32_t steps, double *ms, double *kernel_ms, size_t kernel_count) {

@@ -4,16 +4,16 @@ loss on one tracked particle, which then dominates its CTA's velocity adjoints,
 and particles too far apart for their CTA's box to fit the tile.
 
 Checked against central differences of the f64 oracle (1e-3 relative, the bar
-of the other adjoint tests) and between checkpoint intervals, which decide what
-the adjoint replays beside its sweep and must change the gradients only by the
-f32 order of the node sums: 1e-7 relative per sum, over 2 x SUBSTEPS substeps
-below 1e-5 of the largest component."""
+of the other adjoint tests), between checkpoint intervals, which decide what the
+adjoint replays beside its sweep, and whole against kernel by kernel; these
+must change the gradients only by the f32 order of the node sums: 1e-7 relative
+per sum, over 2 x SUBSTEPS substeps below 1e-5 of the largest component."""
 
 import numpy as np
 import pytest
 
 from oracle import oracle as O
-from tessera_b200 import scenes
+from tessera_b200 import _native, scenes
 from tessera_b200._abi import MAT_ELASTIC, density_particles, make_params
 from tessera_b200.adjoint import Rollout
 
@@ -51,12 +51,16 @@ def check_gradients(params, parts, dt, tracked, seed):
     ref = None
     for every in (SUBSTEPS, 1, 2, 5):
         sim = Rollout(params, parts, dt, SUBSTEPS, checkpoint_every=every)
-        for _ in range(2):  # the second pass replays the captured launches
-            sim.forward(v0, E)
-            got = sim.backward(weight)
-            ref = ref or got
-            for a, b in zip(got, ref):
-                assert np.abs(a - b).max() <= 1e-5 * np.abs(b).max(), every
+        for stepwise in (False, True):
+            if stepwise:
+                assert _native.lib().tmpm_debug_rollout_whole(sim._h) == 3  # both sweeps were one launch
+                _native.lib().tmpm_debug_rollout_stepwise(sim._h)
+            for _ in range(2):  # the second pass replays the captured launches
+                sim.forward(v0, E)
+                got = sim.backward(weight)
+                ref = ref or got
+                for a, b in zip(got, ref):
+                    assert np.abs(a - b).max() <= 1e-5 * np.abs(b).max(), (every, stepwise)
         sim.close()
 
     gv, gE = ref

@@ -10,7 +10,7 @@ import numpy as np
 import pytest
 
 from oracle import oracle as O
-from tessera_b200 import scenes
+from tessera_b200 import _native, scenes
 from tessera_b200.adjoint import Rollout
 
 pytestmark = pytest.mark.gpu
@@ -26,6 +26,7 @@ def gradients(sc, parts, every):
         x, v = sim.forward(parts.velocity, E)
         g = 2.0 * (x.mean(0) - np.asarray(sc.info["target"])) / n
         out.append((x, v) + sim.backward(np.tile(g, (n, 1))))
+    assert _native.lib().tmpm_debug_rollout_whole(sim._h) == 3  # both sweeps ran as one launch
     sim.close()
     return E, out
 

@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 from oracle import oracle as O
-from tessera_b200 import scenes
+from tessera_b200 import _native, scenes
 from tessera_b200._abi import MAT_ELASTIC, MAT_FLUID, ParticleArrays, density_particles, make_params
 from tessera_b200.batch import Batch
 from tessera_b200.session import Session
@@ -25,6 +25,14 @@ def block(count, material, prm, seed=1):
     F = np.eye(3) + rng.uniform(-0.02, 0.02, (count, 3, 3))
     p.deformation[:] = F.transpose(0, 2, 1).reshape(count, 9)
     return p
+
+
+def assert_whole(sim):
+    """Every segment of the session or batch ran as one launch."""
+    L = _native.lib()
+    fn = L.tmpm_debug_batch_segments if isinstance(sim, Batch) else L.tmpm_debug_session_segments
+    whole, stepwise = _native.segment_launches(fn, sim._h)
+    assert whole > 0 and stepwise == 0, (whole, stepwise)
 
 
 def check(cpu, got, steps):
@@ -46,6 +54,7 @@ def test_segment_tracks_the_oracle_at_chunk_edges(shape, count):
         for _ in range(steps):
             cpu.substep_fixed(1e-4)
     check(cpu, s.particles(), 12)
+    assert_whole(s)
 
 
 @pytest.mark.parametrize("steps", [1, 2, 3, 17])
@@ -67,6 +76,7 @@ def test_fluid_deformation_survives_segment_ends(steps):
             cpu.substep_fixed(5e-5)
         got = s.particles()
     check(cpu, got, 2 * steps)
+    assert_whole(s)
     assert np.allclose(got.deformation[3], fluid.deformation[3], atol=1e-7)  # a fixed particle keeps its F
 
 
@@ -84,6 +94,7 @@ def test_fluid_deformation_of_uneven_batch_scenes():
         for _ in range(2 * steps[sid]):
             cpu.substep_fixed(5e-5)
         check(cpu, batch.particles(sid), 2 * steps[sid])
+    assert_whole(batch)
 
 
 def test_sessions_of_several_threads_share_the_gpu():
@@ -101,8 +112,9 @@ def test_sessions_of_several_threads_share_the_gpu():
             s.submit_steps(16)
         s.synchronize()
         out[k] = s.particles()
+        sessions.append(s)
 
-    alone, together = [None] * 3, [None] * 3
+    alone, together, sessions = [None] * 3, [None] * 3, []
     for k, sc in enumerate(made):
         frames(sc, alone, k)
     threads = [threading.Thread(target=frames, args=(sc, together, k)) for k, sc in enumerate(made)]
@@ -110,6 +122,8 @@ def test_sessions_of_several_threads_share_the_gpu():
         t.start()
     for t in threads:
         t.join()
+    for s in sessions:
+        assert_whole(s)
     for a, b in zip(alone, together):
         # 192 substeps apart only by the order of the f32 node sums
         assert np.abs(a.position - b.position).max() < 4e-5
