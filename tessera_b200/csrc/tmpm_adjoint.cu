@@ -869,17 +869,22 @@ __global__ void __launch_bounds__(kTileThreads, 2) k_p2g_back(AdjParams P, Const
 // separated by grid-wide barriers, and the node passes visit only the part of
 // the array the substep's P2G wrote (NodeBounds), which they also clear.
 // Measured before (kernel by kernel, lattice order, sums node by node) and now,
-// host share included: 64,000 particles x 256 substeps forward 9.4 -> 5.2 ms,
-// adjoint 12.0 -> 8.5 ms (stepwise, see kWholeBackward); 4,096 x 64 forward 1.50 ->
-// 0.70, adjoint 1.92 -> 1.18 ms.
+// wall clock of the call in a loop of calls, host share included: 64,000
+// particles x 256 substeps forward 9.4 -> 5.2 ms, adjoint 12.0 -> 8.5 ms (stepwise,
+// see whole_backward_particles); 4,096 x 64 forward 1.50 -> 0.66, adjoint 1.92 ->
+// 1.20 ms.  The same kernels and row order launched one by one: forward 6.0 and 1.06
+// ms, adjoint of 4,096 particles 1.57 ms.
 constexpr int kRolloutThreads = 128;  // 4 CTAs an SM at 128 registers: 75,776 particles on 148 SMs
 
-// Up to here the adjoint is one launch, above it the stepwise sweep with the
-// segment replay on a second stream: two CTAs an SM (measured, 96 substeps, with
-// the host's share: 32,768 particles 2.51 ms whole and 2.74 stepwise, 64,000 3.51
-// and 3.39; 4,096 1.75 and 2.37).  The forward has no replay to overlap and stays
-// whole up to its room.
-constexpr size_t kWholeBackward = 2 * 148 * kRolloutThreads;
+// Up to this many particles the adjoint is one launch, above it the stepwise
+// sweep with the segment replay on a second stream: two CTAs an SM.  Whole against
+// stepwise in ms, 96 substeps, with the host's share: 512 particles 1.75 / 2.18,
+// 4,096 1.75 / 2.37, 17,576 1.99 / 2.53, 32,768 2.49 / 2.71; with three CTAs on some
+// SMs the two are within 4 % (39,304 3.02 / 3.08, 46,656 3.00 / 3.14, 54,872 3.15 /
+// 3.23), with four the stepwise sweep is ahead or level (64,000 3.45 / 3.38, 74,088
+// 3.72 / 3.74).  The forward has no replay to overlap and stays whole up to its
+// room (74,088: 2.57 / 2.75).
+size_t whole_backward_particles() { return static_cast<size_t>(2 * device_sm_count()) * kRolloutThreads; }
 
 struct RolloutArgs {
     const float *E;
@@ -1587,7 +1592,7 @@ TmpmStatus tmpm_adjoint_create(const TmpmParams *params, const TmpmParticleArray
         return TMPM_ERR_DEVICE;
     }
     a->whole_forward = n <= TmpmAdjoint::whole_room(k_rollout_forward<kRolloutThreads>);
-    a->whole_backward = n <= std::min(kWholeBackward, TmpmAdjoint::whole_room(k_rollout_backward<kRolloutThreads>));
+    a->whole_backward = n <= std::min(whole_backward_particles(), TmpmAdjoint::whole_room(k_rollout_backward<kRolloutThreads>));
     a->order = rollout_order(w, P, kRolloutThreads);
     a->each_range([&](size_t begin, size_t end) {
         for (size_t j = begin; j < end; ++j) {

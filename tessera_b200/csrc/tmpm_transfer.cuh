@@ -448,7 +448,9 @@ __device__ __forceinline__ int record_tag(int step_index) { return 1 + (step_ind
 // Added to the tag of a chunk whose particles are near an obstacle: the fast
 // kernel would defer it whole, to run after it; with this bit the chunk is on the
 // no-record list, and the general path runs it beside the fast kernel (with its
-// record).  529k-particle dam break against a sphere, 32 substeps: 2.86 -> 2.28 ms.
+// record).  32 substeps of the 519k-particle dam break against a sphere, launch
+// shape fixed: 2.15 -> 2.09 ms while the flow arrives, 2.53 -> 2.11 ms once it
+// surrounds the sphere; 1.45M particles 4.81 -> 4.84 and 5.31 -> 4.94 ms.
 constexpr int kRecordNear = 4;
 
 #define TMPM_TRANSFER_PARAMS \
