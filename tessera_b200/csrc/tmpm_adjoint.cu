@@ -874,7 +874,7 @@ __global__ void __launch_bounds__(kTileThreads, 2) k_p2g_back(AdjParams P, Const
 // see whole_backward_particles); 4,096 x 64 forward 1.50 -> 0.66, adjoint 1.92 ->
 // 1.20 ms.  The same kernels and row order launched one by one: forward 6.0 and 1.06
 // ms, adjoint of 4,096 particles 1.57 ms.
-constexpr int kRolloutThreads = 128;  // 4 CTAs an SM at 128 registers: 75,776 particles on 148 SMs
+constexpr int kRolloutThreads = 128;  // 4 CTAs an SM at 128 registers: 74,496 particles on 148 SMs
 
 // Up to this many particles the adjoint is one launch, above it the stepwise
 // sweep with the segment replay on a second stream: two CTAs an SM.  Whole against
@@ -1189,7 +1189,7 @@ struct TmpmAdjoint {
             cudaGetLastError();
             return 0;
         }
-        return static_cast<size_t>(per_sm) * device_sm_count() * kRolloutThreads;
+        return static_cast<size_t>(whole_launch_room(per_sm * device_sm_count())) * kRolloutThreads;
     }
 
     // The forward sweep, kernel by kernel: `substeps` substeps from the initial

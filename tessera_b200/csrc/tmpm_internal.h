@@ -67,9 +67,16 @@ constexpr int config_shape(int c) { return c % kNumLaunchShapes; }
 constexpr int config_block_shift(int c) { return c < kNumLaunchShapes ? kBlockShift : kBigBlockShift; }
 // A whole-segment kernel runs up to this many threads an SM (128 registers each,
 // which the general path needs) and takes a scene whose chunks are all resident
-// at once: 75,776 particles on 148 SMs.  Above, kernel by kernel is faster
-// (85,184 particles: 30.1 us a substep against 34.1 with two chunks a CTA).
+// at once (whole_launch_room): 74,496 particles on 148 SMs.  Above, kernel by
+// kernel is faster (85,184 particles: 30.1 us a substep against 34.1 with two
+// chunks a CTA).
 constexpr int kSegmentThreads = 512;
+// Of the CTAs that fit the device at once, how many a whole-segment or whole-rollout
+// launch may take.  Its CTAs fill their SMs, so one that held every SM kept other
+// streams' kernels waiting for its end, where they used to run between its
+// kernels: reading another scene during a batch of 75,600 particles (296 of 296
+// CTAs) took 1.62 ms of its 2.35, 0.06 ms with a few CTAs' room left.
+constexpr int whole_launch_room(int resident) { return resident - (resident + 63) / 64; }
 // It launches at least this many threads: the grid update of a few chunks would
 // otherwise walk its blocks with a few hundred (512 particles 12.1 -> 11.4 us a
 // substep, 11.8 -> 10.5 with CTAs of 128; 37,888 threads give it back to the

@@ -1349,7 +1349,7 @@ void launch_transfer_variant(int mode, const ParticleSoA &P, int n, const DevCla
 }
 
 namespace {
-// Launch k_segment if every chunk has a CTA resident at once.
+// Launch k_segment if every chunk has a CTA resident at once and some are left for other streams.
 template <bool PL, int V, int T, int BS>
 bool try_segment(const ParticleSoA &P, int n, const DevClass *classes, const GridTable &cur, const GridTable &next,
                  const SimParams &sp, const DevObstacle *obstacles, const float *planes, double *reactions,
@@ -1362,7 +1362,7 @@ bool try_segment(const ParticleSoA &P, int n, const DevClass *classes, const Gri
         cudaGetLastError();
         return false;
     }
-    const int room = per_sm * device_sm_count();
+    const int room = whole_launch_room(per_sm * device_sm_count());
     if (chunks > room) return false;
     void *args[] = {const_cast<ParticleSoA *>(&P), &n, &classes, const_cast<GridTable *>(&cur),
                     const_cast<GridTable *>(&next), const_cast<SimParams *>(&sp), &obstacles, &planes, &reactions,

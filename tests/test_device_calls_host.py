@@ -185,3 +185,25 @@ for steps in (16, 2, 16):
             assert count(done, "kernel", "k_grid") == steps, done
 assert s.substeps() == 34 and b.substeps(scene) == 34
 """)
+
+
+def test_whole_segments_leave_room_for_other_streams(run):
+    """A segment that held every SM until its end would keep a read of another scene
+    waiting; with 2 x 148 CTAs resident at once, five are left (rounded up from 1/64)."""
+    run("""
+from tessera_b200._abi import MAT_ELASTIC, density_particles, make_params
+from tessera_b200.batch import Batch
+from tessera_b200.session import Session
+h = 1 / 64
+params = make_params(h, bounds=((0, 0, 0), (1, 1, 1)))
+pos = scenes.lattice((0.2, 0.2, 0.2), (0.55, 0.55, 0.55), h / 2, np.random.default_rng(0), 0.5)
+pos = np.concatenate([pos, pos + 1e-3])
+for count, whole in ((291 * 256, 1), (291 * 256 + 1, 0)):
+    assert len(pos) >= count
+    p = density_particles(pos[:count], h / 4, 1000.0, MAT_ELASTIC, (5e3, 0.3))
+    s, b = Session(params, p, 1e-4, launch_shape=0), Batch(launch_shape=0)
+    s.submit_steps(2)
+    b.submit({b.add_scene(params, p, 1e-4): 2})
+    for sim, fn in ((s, L.tmpm_debug_session_segments), (b, L.tmpm_debug_batch_segments)):
+        assert _native.segment_launches(fn, sim._h) == (whole, 1 - whole), (count, sim)
+""")
